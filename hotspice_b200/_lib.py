@@ -81,6 +81,8 @@ SIGNATURES = {
     'hs_philox_uniform': (C.c_int, [C.c_uint64, C.c_uint64, C.c_int32, P, P]),
     'hs_dipolar_update': (C.c_int, [C.POINTER(HsLattice), C.POINTER(HsSwitchList), P, C.c_int32, C.c_int32, P, P]),
     'hs_dipolar_full_direct': (C.c_int, [C.POINTER(HsLattice), C.c_int32, P, P, P]),
+    'hs_fft_scratch_bytes': (C.c_int64, [C.POINTER(HsLattice)]),
+    'hs_dipolar_full_fft': (C.c_int, [C.POINTER(HsLattice), P, C.c_int64, P, P, P]),
     'hs_igemm_scratch_bytes': (C.c_int64, [C.POINTER(HsLattice), C.c_int32]),
     'hs_dipolar_full_igemm': (C.c_int, [C.POINTER(HsLattice), C.c_int32, P, C.c_int64, P]),
     'hs_set_wait_limit': (C.c_int, [C.c_uint64]),

@@ -70,8 +70,8 @@ class SimParams:
 class EngineConfig:
     """Engine knobs that are not part of the reference's SimParams."""
     resync_every: int = 0          # full dipolar recompute every N progress() steps (0: never)
-    recompute: str = 'auto'        # 'auto' | 'direct64' | 'direct32' | 'igemm'
-    direct_max_pairs: float = 4e11 # 'auto' uses the FP64 direct sum up to this many (cell, window) pairs
+    recompute: str = 'auto'        # 'auto' | 'fft64' | 'direct64' | 'direct32' | 'igemm'
+    direct_max_pairs: float = 4e11 # 'auto' sums in FP64 (fft64, else direct64) up to this many (cell, window) pairs
     persistent: bool = True        # run()/progress() as one persistent cluster launch (hs_engine_run)
     cluster_size: int = 0          # CTAs per cluster for the persistent launch (0: cost model)
     use_graphs: bool = True        # otherwise: replay progress() chunks from captured CUDA graphs
@@ -824,11 +824,28 @@ class Magnets(ABC):
         ks = d.kernel_set
         N = self.nx * self.ny
         W = N if ks.full else (2 * ks.wx + 1) * (2 * ks.wy + 1)
+        nfft = 0
         if method == 'auto':
-            method = 'direct64' if N * W <= self.engine.direct_max_pairs or not self._igemm_ok(d) else 'igemm'
+            method = 'igemm'
+            if N * W <= self.engine.direct_max_pairs or not self._igemm_ok(d):
+                # FP64 either way. The direct sum walks a cell's window serially (about 0.2 us per
+                # entry), so up to 9 x 9 entries it is done before the convolution's three passes
+                # (200 x 200 cells, 5 x 5: 12 against 30 us; 128 x 128, 17 x 17: 55 against 26 us).
+                nfft = self._lib.hs_fft_scratch_bytes(L) if W > 81 else 0
+                method = 'fft64' if nfft > 0 else 'direct64'
+        elif method == 'fft64':
+            nfft = self._lib.hs_fft_scratch_bytes(L)
+            if nfft <= 0:
+                raise ValueError('fft64 recompute: the lattice and its window are longer than the transforms')
         elif method == 'igemm' and not self._igemm_ok(d):
             raise ValueError('igemm recompute needs the full uncropped kernel and a uniform moment')
-        if method == 'direct64':
+        if method == 'fft64':
+            # stream-ordered temporary: the allocator hands the memory on in this stream's order
+            tmp = torch.empty(nfft, device=self.device, dtype=torch.uint8)
+            _lib.check(self._lib.hs_dipolar_full_fft(L, tmp.data_ptr(), nfft, d._E.data_ptr(),
+                                                     _ptr(d._Ep) if self.USE_PERP_ENERGY else None,
+                                                     self._stream()), 'hs_dipolar_full_fft')
+        elif method == 'direct64':
             _lib.check(self._lib.hs_dipolar_full_direct(L, 1, d._E.data_ptr(),
                                                         _ptr(d._Ep) if self.USE_PERP_ENERGY else None,
                                                         self._stream()), 'hs_dipolar_full_direct')

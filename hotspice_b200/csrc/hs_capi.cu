@@ -163,6 +163,21 @@ int hs_dipolar_full_direct(const HsLattice *L, int32_t fp64, double *E64, double
     return hs_launch_dipolar_full_direct(*L, fp64, E64, Ep64, (cudaStream_t)stream);
 }
 
+int64_t hs_fft_scratch_bytes(const HsLattice *L) {
+    if (check_lattice(L, "hs_fft_scratch_bytes") || !L->has_dipolar) return -1;
+    return hs_fft_scratch(*L);
+}
+
+int hs_dipolar_full_fft(const HsLattice *L, void *scratch, int64_t scratch_bytes, double *E64, double *Ep64,
+                        void *stream) {
+    int rc = check_lattice(L, "hs_dipolar_full_fft");
+    if (rc) return rc;
+    if (!L->has_dipolar) { hs_set_error("hs_dipolar_full_fft: lattice has no dipolar energy"); return HS_EINVAL; }
+    if (L->use_perp && !L->Kps) { hs_set_error("hs_dipolar_full_fft: missing perp-self kernels"); return HS_EINVAL; }
+    if (!scratch || !E64 || (L->use_perp && !Ep64)) { hs_set_error("hs_dipolar_full_fft: missing buffer"); return HS_EINVAL; }
+    return hs_launch_dipolar_full_fft(*L, scratch, scratch_bytes, E64, Ep64, (cudaStream_t)stream);
+}
+
 int64_t hs_igemm_scratch_bytes(const HsLattice *L, int32_t nsplit) {
     if (check_lattice(L, "hs_igemm_scratch_bytes")) return -1;
     return hs_igemm_scratch(*L, nsplit);

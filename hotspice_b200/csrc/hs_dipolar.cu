@@ -15,6 +15,7 @@
 // switches on its sublattice, hotspice/energies.py:343-353) contributes only the
 // (2k+1)^2 crop of its kernel with wrap (PBC) or zero fill, like convolve2d(..., 'same').
 #include "hs_common.cuh"
+#include "hs_full.cuh"
 #include "hs_internal.h"
 
 #include "hs_steps.cuh"
@@ -523,38 +524,7 @@ __global__ void dip_full_direct_kernel(HsLattice L, int fp64, double *E64, doubl
         const int s = hs_sub(L, y, x);
         const int mi = L.m[i];
         Acc acc = 0, accp = 0;
-        if (s >= 0 && mi != 0) {
-            if (FULLWIN) {
-                for (int jy = 0; jy < L.ny; ++jy) {
-                    const int dy = jy - y;
-                    const int64_t jrow = (int64_t)jy * L.nx;
-                    for (int jx = 0; jx < L.nx; ++jx) {
-                        const Acc mj = (Acc)L.mm[jrow + jx];
-                        if (mj == (Acc)0) continue;
-                        acc += (Acc)hs_kval(L, L.K, s, dy, jx - x) * mj;
-                        if (L.use_perp) accp += (Acc)hs_kval(L, L.Kps, s, dy, jx - x) * mj;
-                    }
-                }
-            } else {
-                for (int dy = -L.dip_wy; dy <= L.dip_wy; ++dy) {
-                    int jy = y + dy;
-                    if (L.dip_wrap) jy = hs_wrap(jy, L.ny);
-                    else if (jy < 0 || jy >= L.ny) continue;
-                    const int64_t jrow = (int64_t)jy * L.nx;
-                    for (int dx = -L.dip_wx; dx <= L.dip_wx; ++dx) {
-                        int jx = x + dx;
-                        if (L.dip_wrap) jx = hs_wrap(jx, L.nx);
-                        else if (jx < 0 || jx >= L.nx) continue;
-                        const Acc mj = (Acc)L.mm[jrow + jx];
-                        if (mj == (Acc)0) continue;
-                        const int64_t k = (int64_t)s * (2 * L.dip_wy + 1) * (2 * L.dip_wx + 1) +
-                                          (int64_t)(dy + L.dip_wy) * (2 * L.dip_wx + 1) + (dx + L.dip_wx);
-                        acc += (Acc)__ldg(L.K + k) * mj;
-                        if (L.use_perp) accp += (Acc)__ldg(L.Kps + k) * mj;
-                    }
-                }
-            }
-        }
+        if (s >= 0 && mi != 0) dip_full_cell<Acc, FULLWIN>(L, s, y, x, acc, accp);
         const Acc scale = (Acc)L.dip_pref * (Acc)L.moment[i] * (Acc)mi;
         double *Eo = E64 ? E64 : L.E_dip, *Epo = Ep64 ? Ep64 : L.E_dip_perp;
         Eo[i] = (double)(scale * acc);

@@ -15,6 +15,9 @@ int hs_check_launch(const char *what);
 int hs_launch_dipolar_update(const HsLattice &L, const HsSwitchList &sw, const int32_t *n_sw_dev, int n_host,
                              int semantics, const HsCounters *C, cudaStream_t st);
 int hs_launch_dipolar_full_direct(const HsLattice &L, int fp64, double *E64, double *Ep64, cudaStream_t st);
+int64_t hs_fft_scratch(const HsLattice &L);
+int hs_launch_dipolar_full_fft(const HsLattice &L, void *scratch, int64_t scratch_bytes, double *E64, double *Ep64,
+                               cudaStream_t st);
 int64_t hs_neel_scratch(const HsLattice &L);
 int hs_launch_neel(const HsLattice &L, HsCounters *C, const HsSwitchList &sw, double attempt_freq,
                    void *scratch, int64_t scratch_bytes, cudaStream_t st);

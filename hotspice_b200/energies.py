@@ -243,9 +243,10 @@ class DipolarEnergy(Energy):
         return self.mm.unitcell
 
     def update(self, method: str | None = None):
-        """Full recompute (hotspice/energies.py:290-308). ``method``: 'direct64' (FP64
-        direct sum, the default up to EngineConfig.direct_max_pairs cell pairs), 'direct32',
-        or 'igemm' (split-BF16 tensor-core implicit GEMM)."""
+        """Full recompute (hotspice/energies.py:290-308). ``method``: 'fft64' (FP64 fast
+        convolution, the default up to EngineConfig.direct_max_pairs cell pairs), 'direct64'
+        (FP64 direct sum, the default for windows of a few cells), 'direct32', or 'igemm'
+        (split-BF16 tensor-core implicit GEMM)."""
         self.mm._full_recompute(self, method)
 
     def update_single(self, index2D):

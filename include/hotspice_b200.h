@@ -11,6 +11,7 @@
  *   hs_dipolar_update        DipolarEnergy.update_single / update_multiple
  *                            (hotspice/energies.py:310-329, 331-366)
  *   hs_dipolar_full_direct   DipolarEnergy.update (hotspice/energies.py:290-308), direct sum
+ *   hs_dipolar_full_fft      DipolarEnergy.update as a fast convolution in FP64
  *   hs_dipolar_full_igemm    DipolarEnergy.update as a tensor-core implicit GEMM
  *   hs_neel_step             Magnets._update_Néel + E_barrier + update_energy
  *                            (hotspice/core.py:679-709, 625-656, 241-253)
@@ -208,6 +209,15 @@ int hs_dipolar_update(const HsLattice *L, const HsSwitchList *sw, const int32_t 
 /* Direct sum over the kernel window. fp64 != 0 accumulates in double, otherwise in float.
  * Writes E64/Ep64 when given, else L->E_dip / L->E_dip_perp. */
 int hs_dipolar_full_direct(const HsLattice *L, int32_t fp64, double *E64, double *Ep64, void *stream);
+/* The same sums as a fast convolution in FP64 (they differ from the direct sum's by FP64
+ * rounding; sums below the rounding of their largest possible terms are 0). Every window form:
+ * uncut, cropped, minimum-image. hs_fft_scratch_bytes: the scratch it needs, 0 when the lattice
+ * plus its window is longer than the transforms (4096 cells along an axis; lattice plus twice the
+ * window with minimum-image wrapping). Writes E64, and Ep64 with use_perp. The scratch needs no
+ * initial value and holds nothing between calls. */
+int64_t hs_fft_scratch_bytes(const HsLattice *L);
+int hs_dipolar_full_fft(const HsLattice *L, void *scratch, int64_t scratch_bytes, double *E64, double *Ep64,
+                        void *stream);
 /* Tensor-core implicit GEMM (tcgen05, split-BF16 kernel, FP32 accumulation in TMEM), the
  * counterpart of DipolarEnergy.update (hotspice/energies.py:290-308) for the full, uncropped
  * kernel (dip_wx = nx-1, dip_wy = ny-1, no wrap) and a uniform moment over the occupied cells.
