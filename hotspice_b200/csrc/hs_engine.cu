@@ -527,7 +527,7 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
         if (!sh.go[st & 1]) break;
         if (scheme == HS_SCHEME_METROPOLIS) {
             if (rank == 0) {
-                metro_step_cta(L, C, sw, P, metro_scratch_of(L, P, I.scratch), ws_bytes > 0 ? s_ws : nullptr,
+                metro_step_cta<true>(L, C, sw, P, metro_scratch_of(L, P, I.scratch), ws_bytes > 0 ? s_ws : nullptr,
                                ws_bytes);
                 __syncthreads();
                 if (threadIdx.x == 0) { S.publish(&sh.nsw, C->n_sw); decide_next(st + 1); }

@@ -17,10 +17,14 @@
 
 namespace {
 
-__global__ void __launch_bounds__(MT) metropolis_kernel(HsLattice L, HsCounters *C, HsSwitchList sw, HsGridPlan P,
+// MT threads; Poisson-disc plans take PT, whose sampler needs few threads and more than the 64
+// registers that MT leaves each.
+constexpr int PT = 512;
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) metropolis_kernel(HsLattice L, HsCounters *C, HsSwitchList sw, HsGridPlan P,
                                                         MetroScratch S, int ws_bytes) {
     extern __shared__ __align__(16) unsigned char s_ws[];   // the Poisson-disc sampler's arrays, if given
-    metro_step_cta(L, C, sw, P, S, ws_bytes > 0 ? s_ws : nullptr, ws_bytes);
+    metro_step_cta<THREADS == PT>(L, C, sw, P, S, ws_bytes > 0 ? s_ws : nullptr, ws_bytes);
 }
 
 constexpr int64_t METRO_WS_MAX = 200 * 1024;   // dynamic shared memory the Poisson sampler may use
@@ -64,12 +68,13 @@ int hs_launch_metropolis(const HsLattice &L, HsCounters *C, const HsSwitchList &
         ws = (int)hs_poisson_mem_bytes(gsz);
         static int granted = 0;
         if (ws > 48 * 1024 && ws > granted) {
-            cudaError_t e = cudaFuncSetAttribute(metropolis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)METRO_WS_MAX);
+            cudaError_t e = cudaFuncSetAttribute(metropolis_kernel<PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)METRO_WS_MAX);
             if (e != cudaSuccess) { hs_set_error("metropolis_kernel: %s", cudaGetErrorString(e)); return HS_ECUDA; }
             granted = (int)METRO_WS_MAX;
         }
     }
-    metropolis_kernel<<<1, MT, ws, st>>>(L, C, sw, P, S, ws);
+    if (P.sample_scheme == HS_SAMPLE_POISSON) metropolis_kernel<PT><<<1, PT, ws, st>>>(L, C, sw, P, S, ws);
+    else metropolis_kernel<MT><<<1, MT, 0, st>>>(L, C, sw, P, S, 0);
     int rc = hs_check_launch("metropolis_kernel");
     if (rc) return rc;
     if (L.has_dipolar) return hs_launch_dipolar_update(L, sw, &C->n_sw, 0, HS_UPDATE_MULTIPLE, C, st);

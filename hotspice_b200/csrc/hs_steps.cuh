@@ -133,8 +133,8 @@ HS_DEV PoissonMem poisson_mem_in(void *base, int gsz) {
 }
 
 // Poisson-disc dart throwing in cell units (hotspice/poisson.py:72-128 restated in cells),
-// executed by one warp. Returns the number of points written to (S.py, S.px) as nearest cell
-// indices and advances `call` by the variates consumed.
+// executed by one warp, for any number of tries K; poisson_block is the form for the usual one.
+// Returns the number of points, and advances `call` by the variates consumed.
 // Bridson's loop is sequential over active points, but the k tries of one active point always
 // consume 1 + 2k variates (queue pick, then angle and distance of each try), so the warp
 // evaluates the k candidates at once (lane t: try t) and their 5x5-cell conflict checks against
@@ -154,7 +154,6 @@ HS_DEV int poisson_warp(const HsLattice &L, const HsGridPlan &P, const MetroScra
     const int gw = (int)ceil(width / cs), gh = (int)ceil(height / cs);
     const int gsz = gw * gh;
     const int K = P.poisson_k;
-    if (gsz > S.gsz || K < 1 || 25 * K > 32 * 32) { if (lane == 0) *status |= HS_ST_POISSON_OVERFLOW; return 0; }
     for (int g = lane; g < gsz; g += 32) M.grid[g] = -1;
     __syncwarp();
     auto rnd_at = [&](uint64_t c) { return hs_u53(L.seed, c, 0u); };
@@ -252,34 +251,244 @@ HS_DEV int poisson_warp(const HsLattice &L, const HsGridPlan &P, const MetroScra
     }
     if (overflow && lane == 0) *status |= HS_ST_POISSON_OVERFLOW;
     __syncwarp();
-    // keep points with x < max(r, w - r), y < max(r, h - r) (PBC=True default), then offset;
-    // in grid-cell order, compacted by the warp
+    return npts;
+}
+
+constexpr int POISSON_K = 4;                        // tries per active point of the block form
+constexpr int POISSON_BATCH = 32;                   // active points whose variates are made together
+constexpr int POISSON_PROD = POISSON_K * POISSON_BATCH;   // producer threads
+
+// Work arrays of poisson_block in the same shared memory (24 bytes per background cell): the point
+// in each cell, or POISSON_EMPTY; the cell of each point number; the active numbers as a bitmap.
+constexpr double POISSON_EMPTY = 1e300;             // farther than any radius
+struct PoissonCells {
+    double2 *pos;
+    int32_t *cell_of;
+    unsigned *words;
+};
+HS_DEV PoissonCells poisson_cells_in(unsigned char *base, int gsz) {
+    PoissonCells M;
+    M.pos = reinterpret_cast<double2 *>(base);
+    M.cell_of = reinterpret_cast<int32_t *>(M.pos + gsz);
+    M.words = reinterpret_cast<unsigned *>(M.cell_of + gsz);
+    return M;
+}
+
+// The loop of poisson_warp for K = POISSON_K on the dynamic shared memory of a CTA of at least
+// 32 + POISSON_PROD threads: the points, their order and the variates are the same. An active
+// point's variates depend only on how many points came before it, so warps 1-4 make the next 32
+// points' variates, sines and distances while warp 0 runs the sequential part, which has no
+// transcendental left. The queue is the set of active point numbers in order (appended in order,
+// popped anywhere), so it is a bitmap and the pick the qi-th set bit; eight lanes per try check
+// its 25 cells, and the tries' mutual conflicts are tested in parallel. The chain of one point is
+// bound by its instructions' latencies (loads, shuffles and ballots of 30 cycles each, one warp):
+// about 1,600 cycles against 3,000 for poisson_warp on one warp. The selection kernel at 1024^2,
+// r = 84 cells, about 65 points a step: 203 -> 61 us.
+HS_DEV int poisson_block(const HsLattice &L, const HsGridPlan &P, int cap, uint64_t call0, int *n_iter, int *status) {
+    extern __shared__ __align__(16) unsigned char s_ws[];
+    __shared__ double s_u[2][POISSON_BATCH], s_d[2][POISSON_PROD], s_c[2][POISSON_PROD], s_s[2][POISSON_PROD];
+    __shared__ int s_np, s_it, s_more[2];   // s_more: by batch parity, so a late reader never sees the next one
+    constexpr int K = POISSON_K;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const double width = L.nx, height = L.ny;
+    const double r = P.r_cells + 1.0;
+    const double cs = r / sqrt(2.0), inv = 1.0 / cs;
+    const double rSq = r * r;
+    const int gw = (int)ceil(width / cs), gh = (int)ceil(height / cs);
+    const int gsz = gw * gh;
+    const int nw = (gsz + 31) >> 5, cw = (nw + 31) >> 5;   // bitmap words, and words per lane
+    const PoissonCells M = poisson_cells_in(s_ws, gsz);
+    for (int g = threadIdx.x; g < gsz; g += blockDim.x) M.pos[g] = make_double2(POISSON_EMPTY, POISSON_EMPTY);
+    for (int g = threadIdx.x; g < nw; g += blockDim.x) M.words[g] = g == 0 ? 1u : 0u;
+    // (int)(v / cs); the division itself only next to a cell border
+    auto cell = [&](double v) {
+        const double q = v * inv;
+        const int i = (int)q;
+        const double f = q - (double)i;
+        return (f < 1e-6 || f > 1.0 - 1e-6) ? (int)(v / cs) : i;
+    };
+    const bool small = gsz < 4 * gw + 16;       // flat cell numbers may wrap more than once
+    const double hw = width * 0.5, hh = height * 0.5;
+    auto near = [&](double dx, double dy) {     // the distance rule of the grid check
+        dx = fabs(dx);
+        dy = fabs(dy);
+        dx = dx > hw ? dx - width : dx;
+        dy = dy > hh ? dy - height : dy;
+        return dx * dx + dy * dy <= rSq;
+    };
+    auto produce = [&](int batch) {   // threads 32 .. 32 + POISSON_PROD - 1
+        const int e = threadIdx.x - 32, it = e / K, t = e - it * K, b = batch & 1;
+        const uint64_t c = call0 + 2 + (uint64_t)(batch * POISSON_BATCH + it) * (1 + 2 * K);
+        if (t == 0) s_u[b][it] = hs_u53(L.seed, c, 0u);
+        const double alpha = 6.283185307179586 * hs_u53(L.seed, c + 1 + 2 * t, 0u);
+        s_d[b][e] = r * sqrt(3.0 * hs_u53(L.seed, c + 2 + 2 * t, 0u) + 1.0);
+        s_c[b][e] = cos(alpha);
+        s_s[b][e] = sin(alpha);
+    };
+    __syncthreads();
+    if (warp >= 1 && warp <= POISSON_PROD / 32) produce(0);
+    else if (warp == 0 && lane == 0) {
+        const double p0x = (double)(int)(width * hs_u53(L.seed, call0, 0u));
+        const double p0y = (double)(int)(height * hs_u53(L.seed, call0 + 1, 0u));
+        const int c = (int)(p0x / cs) + (int)(p0y / cs) * gw;
+        M.pos[c] = make_double2(p0x, p0y);
+        M.cell_of[0] = c;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int npts = 1, nq = 1, it = 0;
+        // bitmap: lane l counts the set bits of words [l cw, (l + 1) cw) and those before them
+        int cnt = lane == 0 ? 1 : 0, pre = lane == 0 ? 0 : 1;
+        unsigned mine = lane == 0 ? 1u : 0u;               // the lane's word when cw == 1
+        const int own = 32 * cw * lane;                    // the lane's first point number
+        const int t = lane >> 3, sub = lane & 7;
+        int off[4];                                        // the lane's cells of a try's 5 x 5 (the last one again)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { const int c = min(sub + 8 * j, 24); off[j] = (c / 5 - 2) + (c % 5 - 2) * gw; }
+        // pairs of tries u < v, on lanes 0-5: (0,1) (0,2) (1,2) (0,3) (1,3) (2,3)
+        const int lv = lane == 0 ? 8 : (lane < 3 ? 16 : 24), lu = 8 * (lane < 3 ? (lane == 2 ? 1 : 0) : (lane - 3) & 3);
+        bool overflow = false;
+        for (int batch = 0;; ++batch) {
+            const int b = batch & 1;
+            for (int k = 0; k < POISSON_BATCH && nq > 0 && !overflow; ++k, ++it) {
+                const int qi = (int)(s_u[b][k] * nq);
+                const int e = k * K + t;
+                const double d = s_d[b][e], ca = s_c[b][e], sa = s_s[b][e];
+                // the qi-th active point
+                const int src = __ffs(__ballot_sync(0xffffffffu, pre <= qi && qi < pre + cnt)) - 1;
+                int rank = qi - __shfl_sync(0xffffffffu, pre, src);
+                int wi = src;
+                unsigned word;
+                if (cw == 1) word = __shfl_sync(0xffffffffu, mine, src);
+                else {                              // cw < 32: the arrays fit shared memory
+                    const unsigned w = (lane < cw && src * cw + lane < nw) ? M.words[src * cw + lane] : 0u;
+                    const int c = __popc(w);
+                    int inc = c;
+#pragma unroll
+                    for (int s = 1; s < 32; s <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, s); if (lane >= s) inc += v; }
+                    const int sl = __ffs(__ballot_sync(0xffffffffu, inc > rank)) - 1;
+                    rank -= __shfl_sync(0xffffffffu, inc - c, sl);
+                    word = __shfl_sync(0xffffffffu, w, sl);
+                    wi = src * cw + sl;
+                }
+                const int bit = __ffs(__ballot_sync(0xffffffffu, ((word >> lane) & 1u) && __popc(word & below) == rank)) - 1;
+                // try t of this point (the same on its eight lanes) and its cell
+                const double2 q = M.pos[M.cell_of[32 * wi + bit]];
+                word &= ~(1u << bit);
+                if (lane == src) { --cnt; mine = word; }
+                if (lane > src) --pre;
+                if (cw > 1 && lane == 0) M.words[wi] = word;
+                nq -= 1;
+                const double px = q.x + d * ca, py = q.y + d * sa;
+                const bool inb = 0.0 <= px && px < width && 0.0 <= py && py < height;
+                const int flat = inb ? cell(px) + cell(py) * gw : 0;
+                // existing points in the cells around it (branch-free, so that the loads overlap)
+                int g[4];
+                if (small) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) g[j] = pymod(flat + off[j], gsz);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { const int c = flat + off[j]; g[j] = c < 0 ? c + gsz : (c >= gsz ? c - gsz : c); }
+                }
+                double2 h[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) h[j] = M.pos[g[j]];
+                // tries u < v in conflict, u's cell being among those v checks
+                const double ux = __shfl_sync(0xffffffffu, px, lu), uy = __shfl_sync(0xffffffffu, py, lu);
+                const double vx = __shfl_sync(0xffffffffu, px, lv), vy = __shfl_sync(0xffffffffu, py, lv);
+                const int df = __shfl_sync(0xffffffffu, flat, lu) - __shfl_sync(0xffffffffu, flat, lv) + 2;
+                bool hit = !inb;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) hit |= near(px - h[j].x, py - h[j].y);
+                bool pair = near(vx - ux, vy - uy) && lane < 6;
+                if (pair) {                         // (uf - vf - a gw + 2) mod gsz <= 4 for a row a = -2..2
+                    bool seen = false;
+                    for (int a = -2; a <= 2; ++a) seen |= pymod(df - a * gw, gsz) <= 4;
+                    pair = seen;
+                }
+                const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                const unsigned pairs = __ballot_sync(0xffffffffu, pair);
+                unsigned amask = 0u;
+                if (!(hits & 0xffu)) amask = 1u;
+                if (!(hits & 0xff00u) && !(amask & (pairs & 1u))) amask |= 2u;
+                if (!(hits & 0xff0000u) && !(amask & ((pairs >> 1) & 3u))) amask |= 4u;
+                if (!(hits & 0xff000000u) && !(amask & ((pairs >> 3) & 7u))) amask |= 8u;
+                if (amask) {                        // warp-uniform
+                    while (npts + __popc(amask) > cap) { amask &= ~(0x80000000u >> __clz(amask)); overflow = true; }
+                    const int nacc = __popc(amask);
+                    if (sub == 0 && ((amask >> t) & 1u)) {
+                        M.pos[flat] = make_double2(px, py);
+                        M.cell_of[npts + __popc(amask & ((1u << t) - 1u))] = flat;
+                    }
+                    // the new numbers [npts, npts + nacc) are active
+                    const int lo = min(max(npts - own, 0), 32 * cw), hi = min(max(npts + nacc - own, 0), 32 * cw);
+                    cnt += hi - lo;
+                    pre += min(max(own - npts, 0), nacc);
+                    if (cw == 1) mine |= hi > lo ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
+                    else if (lane == 0)
+                        for (int id = npts; id < npts + nacc; ++id) M.words[id >> 5] |= 1u << (id & 31);
+                    npts += nacc;
+                    nq += nacc;
+                }
+                __syncwarp();
+            }
+            const bool more = nq > 0 && !overflow;
+            if (lane == 0) s_more[b] = more;
+            asm volatile("bar.sync 1, %0;" ::"n"(32 + POISSON_PROD) : "memory");   // the next batch is ready
+            if (!more) break;
+        }
+        if (lane == 0) {
+            s_np = npts;
+            s_it = it;
+            if (overflow) *status |= HS_ST_POISSON_OVERFLOW;
+        }
+    } else if (warp <= POISSON_PROD / 32) {
+        for (int batch = 1;; ++batch) {
+            produce(batch);
+            asm volatile("bar.sync 1, %0;" ::"n"(32 + POISSON_PROD) : "memory");
+            if (!s_more[(batch & 1) ^ 1]) break;
+        }
+    }
+    __syncthreads();
+    *n_iter = s_it;
+    return s_np;
+}
+
+// Select from the sampled points, by the whole CTA: those with x < max(r, w - r), y < max(r, h - r)
+// (PBC=True default), offset by the next two variates, in grid-cell order. point(g, x, y) gives the
+// point of background cell g, if there is one. Returns how many nearest cell indices were written to
+// (S.py, S.px).
+template <typename Point>
+HS_DEV int poisson_select(const HsLattice &L, const HsGridPlan &P, const MetroScratch &S, Point point, uint64_t &call,
+                          int *warp_tot, int *status) {
+    const double width = L.nx, height = L.ny;
+    const double r = P.r_cells + 1.0;
+    const double cs = r / sqrt(2.0);
+    const int gsz = (int)ceil(width / cs) * (int)ceil(height / cs);
     const double lx = fmax(r, width - r), ly = fmax(r, height - r);
-    const double ox = (double)(int)(rnd_at(call) * width), oy = (double)(int)(rnd_at(call + 1) * height);
+    const double ox = (double)(int)(hs_u53(L.seed, call, 0u) * width), oy = (double)(int)(hs_u53(L.seed, call + 1, 0u) * height);
     call += 2;
     int k = 0;
-    for (int g0 = 0; g0 < gsz; g0 += 32) {
-        const int g = g0 + lane;
-        const int p = g < gsz ? M.grid[g] : -1;
-        bool keep = false;
+    for (int g0 = 0; g0 < gsz; g0 += blockDim.x) {
+        const int g = g0 + (int)threadIdx.x;
+        double x = 0.0, y = 0.0;
+        bool keep = g < gsz && point(g, x, y);
         int ix = 0, iy = 0;
-        if (p >= 0) {
-            const double x = M.ptx[p], y = M.pty[p];
-            keep = x >= 0.0 && y >= 0.0 && x < lx && y < ly;
-            if (keep) {
-                const double fx = fmod(x + ox, width), fy = fmod(y + oy, height);
-                // nearest cell index, ties to the lower index
-                ix = (int)floor(fx); if (fx - ix > 0.5) ix += 1; ix = min(max(ix, 0), L.nx - 1);
-                iy = (int)floor(fy); if (fy - iy > 0.5) iy += 1; iy = min(max(iy, 0), L.ny - 1);
-            }
+        keep = keep && x >= 0.0 && y >= 0.0 && x < lx && y < ly;
+        if (keep) {
+            const double fx = fmod(x + ox, width), fy = fmod(y + oy, height);
+            // nearest cell index, ties to the lower index
+            ix = (int)floor(fx); if (fx - ix > 0.5) ix += 1; ix = min(max(ix, 0), L.nx - 1);
+            iy = (int)floor(fy); if (fy - iy > 0.5) iy += 1; iy = min(max(iy, 0), L.ny - 1);
         }
-        const unsigned b = __ballot_sync(0xffffffffu, keep);
-        const int pos = k + __popc(b & below);
+        int tot;
+        const int pos = k + block_excl_scan(keep, warp_tot, tot);
         if (keep && pos < S.cap) { S.py[pos] = iy; S.px[pos] = ix; }
-        k += __popc(b);
+        k += tot;
     }
-    if (k > S.cap) { if (lane == 0) *status |= HS_ST_POISSON_OVERFLOW; k = S.cap; }
-    __syncwarp();
+    if (k > S.cap) { if (threadIdx.x == 0) *status |= HS_ST_POISSON_OVERFLOW; k = S.cap; }
     return k;
 }
 
@@ -522,11 +731,12 @@ HS_DEV bool metro_grid_warp(const HsLattice &L, HsCounters *C, const HsSwitchLis
     return true;
 }
 
-// One Metropolis step executed by one CTA (selection, acceptance, flips, switch list).
+// One Metropolis step executed by one CTA (selection, acceptance, flips, switch list). POISSON: the
+// plan may be a Poisson-disc one (a kernel that never sees one leaves the sampler's code out).
+template <bool POISSON>
 HS_DEV void metro_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList &sw, const HsGridPlan &P,
                            const MetroScratch &S, void *ws = nullptr, int ws_bytes = 0) {
     __shared__ int warp_tot[33];
-    __shared__ int s_k;
     __shared__ uint64_t s_call;
     __shared__ int s_status;
     __shared__ int s_bins[256];
@@ -607,21 +817,45 @@ HS_DEV void metro_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
             if (threadIdx.x == 0) { const int f = L.nonzero[i]; S.py[0] = f / L.nx; S.px[0] = f % L.nx; }
             call += 1;
             k = 1;
-        } else {  // Poisson
-            if (threadIdx.x < 32) {
-                uint64_t c = call;
-                int st = 0;
-                // the sampler's arrays in the shared workspace when they fit, else in the scratch
-                const int64_t g = (int64_t)hs_poisson_grid_cells(L, P);
-                PoissonMem M;
-                if (ws && hs_poisson_mem_bytes(g) <= ws_bytes) M = poisson_mem_in(ws, (int)g);
-                else { M.grid = S.grid; M.ptx = S.ptx; M.pty = S.pty; M.queue = S.queue; }
-                const int n = poisson_warp(L, P, S, M, c, &st);
-                if (threadIdx.x == 0) { s_k = n; s_call = c; s_status |= st; }
+        } else if constexpr (POISSON) {
+            // the sampler's arrays in the shared workspace when they fit, else in the scratch
+            const int64_t g = (int64_t)hs_poisson_grid_cells(L, P);
+            if (g > S.gsz || P.poisson_k < 1 || 25 * P.poisson_k > 32 * 32) {   // no samples: retry, then report
+                if (threadIdx.x == 0) s_status |= HS_ST_POISSON_OVERFLOW;
+                k = 0;
+                continue;
             }
-            __syncthreads();
-            k = s_k;
-            call = s_call;
+            const bool fits = ws && hs_poisson_mem_bytes(g) <= ws_bytes;
+            int st = 0;
+            if (fits && P.poisson_k == POISSON_K && blockDim.x >= 32 + POISSON_PROD) {
+                int iters;
+                poisson_block(L, P, S.gsz, call, &iters, &st);
+                call += 2 + (uint64_t)iters * (1 + 2 * POISSON_K);
+                const PoissonCells M = poisson_cells_in(reinterpret_cast<unsigned char *>(ws), (int)g);
+                k = poisson_select(L, P, S, [&](int c, double &x, double &y) {
+                    const double2 p = M.pos[c];
+                    x = p.x; y = p.y;
+                    return p.x < POISSON_EMPTY;
+                }, call, warp_tot, &st);
+            } else {
+                PoissonMem M;
+                if (fits) M = poisson_mem_in(ws, (int)g);
+                else { M.grid = S.grid; M.ptx = S.ptx; M.pty = S.pty; M.queue = S.queue; }
+                if (threadIdx.x < 32) {
+                    uint64_t c = call;
+                    poisson_warp(L, P, S, M, c, &st);
+                    if (threadIdx.x == 0) s_call = c;
+                }
+                __syncthreads();
+                call = s_call;
+                k = poisson_select(L, P, S, [&](int c, double &x, double &y) {
+                    const int p = M.grid[c];
+                    if (p < 0) return false;
+                    x = M.ptx[p]; y = M.pty[p];
+                    return true;
+                }, call, warp_tot, &st);
+            }
+            if (threadIdx.x == 0) s_status |= st;
         }
         __syncthreads();
         // ---- select(): drop unoccupied picks, retry if none is left (core.py:484-487) -------
