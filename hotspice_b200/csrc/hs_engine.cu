@@ -6,7 +6,8 @@
 // step instead of kernel boundaries:
 //   Metropolis: [CTA 0] selection + acceptance + flips (metro_step_cta)  | barrier |
 //               [all]   dipolar update of the touched strips              | barrier |
-//   Néel:       [all]   barrier/log-time keys of a slice of the cells, CTA argmin -> CTA 0
+//   Néel:       on owned cells for a uniform temperature (neel_run_owned); else
+//               [all]   barrier/log-time keys of a slice of the cells, CTA argmin -> CTA 0
 //                       through distributed shared memory                 | barrier |
 //               [CTA 0] final argmin, switching time, flip                | barrier |
 //               [all]   dipolar update                                    | barrier |
@@ -242,13 +243,13 @@ HS_DEV void update_items(const HsLattice &L, const SwX *s_sw, int n, int semanti
     }
 }
 
-// Window update of a single switch (the Néel step): every thread of the cluster takes window
-// cells directly (row-major over the window, consecutive threads on consecutive columns) and
-// issues the loads of its cells together; the barrier cache is refreshed in the same pass. Per
-// cell the arithmetic is that of update_items for one switch (acc = mm_s K, E += 2 pref mm_j acc
-// in the same float order, then E_s negated), so the energies are the same bit for bit; cells
-// outside the window receive nothing there either.
-HS_DEV void update_one(const HsLattice &L, int sy, int sx, float smm, int8_t sm, int t0, int nt, float *cache) {
+// Window update of a single switch (the Néel step without the owner path): every thread of the
+// cluster takes window cells directly (row-major over the window, consecutive threads on
+// consecutive columns) and issues the loads of its cells together. Per cell the arithmetic is that
+// of update_items for one switch (acc = mm_s K, E += 2 pref mm_j acc in the same float order, then
+// E_s negated), so the energies are the same bit for bit; cells outside the window receive nothing
+// there either.
+HS_DEV void update_one(const HsLattice &L, int sy, int sx, float smm, int t0, int nt) {
     const int sub = hs_sub(L, sy, sx);
     if (sub < 0) return;
     int hy, wy, hx, wx;
@@ -270,9 +271,8 @@ HS_DEV void update_one(const HsLattice &L, int sy, int sx, float smm, int8_t sm,
     int r0 = t0 / ncols, q0 = t0 - r0 * ncols;
     for (int base = t0; base < total; base += nt * U) {
         int idx[U], rw[U], cl[U];
-        float kv[U], kp[U], mv[U], zf[U], zp[U], eb[U];
+        float kv[U], kp[U], mv[U];
         double ev[U], pv[U];
-        int8_t oc[U], ms[U];
         bool live[U];   // in the window and on a unit-cell site that holds magnets
 #pragma unroll
         for (int k = 0; k < U; ++k) {
@@ -286,7 +286,7 @@ HS_DEV void update_one(const HsLattice &L, int sy, int sx, float smm, int8_t sm,
             rw[k] = row; cl[k] = col;
             idx[k] = row * L.nx + col;
             // a site without a kernel never holds a magnet: its energy stays 0 (the reference adds
-            // m * ... = 0 there) and the Néel scan never reads its cache entry
+            // m * ... = 0 there)
             live[k] = c < total && hs_sub(L, row, col) >= 0;
         }
 #pragma unroll
@@ -295,19 +295,11 @@ HS_DEV void update_one(const HsLattice &L, int sy, int sx, float smm, int8_t sm,
             const int i = idx[k];
             kv[k] = v ? hs_kval(L, L.K, sub, rw[k] - sy, cl[k] - sx) : 0.f;
             kp[k] = (v && two) ? hs_kval(L, L.Kpo, sub, rw[k] - sy, cl[k] - sx) : 0.f;
-            // the switched cell's new moment and spin come from the handover (smm, sm): its
-            // global writes may still be in flight
-            const bool src = rw[k] == sy && cl[k] == sx;
-            mv[k] = v ? (src ? smm : __ldcg(L.mm + i)) : 0.f;
+            // the switched cell's new moment comes from the handover (smm): its global write may
+            // still be in flight
+            mv[k] = v ? (rw[k] == sy && cl[k] == sx ? smm : __ldcg(L.mm + i)) : 0.f;
             ev[k] = v ? __ldcg(L.E_dip + i) : 0.0;
             pv[k] = (v && two) ? __ldcg(L.E_dip_perp + i) : 0.0;
-            if (cache) {
-                oc[k] = v ? L.occ[i] : (int8_t)0;
-                ms[k] = v ? (src ? sm : __ldcg(L.m + i)) : (int8_t)0;
-                zf[k] = (v && L.zee) ? __ldg(L.zee + i) : 0.f;
-                zp[k] = (v && L.zee && two) ? __ldg(L.zee_perp + i) : 0.f;
-                eb[k] = v ? __ldg(L.E_B + i) : 0.f;
-            }
         }
 #pragma unroll
         for (int k = 0; k < U; ++k) {
@@ -321,16 +313,6 @@ HS_DEV void update_one(const HsLattice &L, int sy, int sx, float smm, int8_t sm,
             if (rw[k] == sy && cl[k] == sx) { e = -e; p = -p; }
             L.E_dip[i] = e;
             if (two) L.E_dip_perp[i] = p;
-            if (cache) {
-                float c = INFINITY;
-                if (oc[k]) {
-                    const double m = (double)ms[k];
-                    double E = e, Ep = p;
-                    if (L.zee) { E += m * (double)zf[k]; if (two) Ep += m * (double)zp[k]; }
-                    c = neel_cache_value(L, E, two ? Ep : 0.0, (double)eb[k]);
-                }
-                cache[i] = c;
-            }
         }
     }
 }
@@ -424,19 +406,26 @@ HS_DEV WolffScratch wolff_scratch_of(const HsLattice &L, void *base) {
     return S;
 }
 
+constexpr int NEEL_OWN_UY = 64;     // rows of a period that the owner path's table holds
+
 // Shared state of one CTA while it runs an instance.
 struct __align__(16) EngShared {
     HsInstance I;                       // the instance descriptor, staged (read through references)
     HsCounters C;                       // rank 0: the instance's counters for the whole run
     unsigned long long call[2];         // Philox call of step st in call[st & 1]
-    HsKeyIdx part[16];
+    HsKeyIdx part[2][16];               // owner path: the CTAs' minima of step st in part[st & 1]
     HsKeyIdx red[32];
     double dred[32];
     int inst, n1, y1, x1, m1, nsw;
     int go[2];                          // step st runs while go[st & 1] (double-buffered)
     float mm1;
-    int nq[ENG_NT / 32][NEEL_QCAP];     // per-warp candidate queues of the cached Néel scan
-    SwX sw[ENG_SWCAP];
+    double thr[2];                      // owner path: a key below thr[st & 1] switches for certain
+    float tw[32];                       // owner path: the warps' bounds
+    int rowpre[NEEL_OWN_UY + 1];        // owner path: occupied cells before row y of a period of uy rows
+    union {
+        struct { int q[ENG_NT / 32][NEEL_QCAP]; float lb[ENG_NT / 32][NEEL_QCAP]; } nq;   // owner path: candidates
+        SwX sw[ENG_SWCAP];
+    };
 };
 static_assert(sizeof(HsInstance) % 8 == 0, "HsInstance is copied in 8-byte words");
 static_assert(sizeof(HsCounters) % 8 == 0, "HsCounters is copied in 8-byte words");
@@ -461,6 +450,22 @@ struct RunSync {
         if (CS == 1 || alone) *local = v;
         else Sync<CS>::publish(local, v);
     }
+    // v into every CTA's copy of *local, one CTA per lane of the calling warp
+    template <typename T>
+    HS_DEV void publish_warp(T *local, T v, int n_cta) const {
+        const int lane = threadIdx.x & 31;
+        if (CS == 1 || alone) { if (lane == 0) *local = v; }
+        else if (lane < n_cta) *cg::this_cluster().map_shared_rank(local, lane) = v;
+    }
+    // *from (in this CTA) into every CTA's copy of *local, 8 bytes per lane of the calling warp
+    template <typename T>
+    HS_DEV void copy_to_all(T *local, const T *from, int n_cta) const {
+        constexpr int NW = sizeof(T) / 8;
+        static_assert(sizeof(T) % 8 == 0, "copied in 8-byte words");
+        const unsigned long long *src = reinterpret_cast<const unsigned long long *>(from);
+        for (int k = threadIdx.x & 31; k < n_cta * NW; k += 32)
+            reinterpret_cast<unsigned long long *>(cg::this_cluster().map_shared_rank(local, k / NW))[k % NW] = src[k % NW];
+    }
     // rank 0's slot r of a per-CTA array receives v (r = this CTA's rank)
     template <typename T>
     HS_DEV void to_rank0(T *arr, int r, T v) const {
@@ -469,6 +474,455 @@ struct RunSync {
         else *cg::this_cluster().map_shared_rank(&arr[r], 0) = v;
     }
 };
+
+// ---- Néel steps with owned cells ---------------------------------------------------------
+// The Néel path for a uniform temperature without exchange (bounds per cell that only a switch in
+// reach changes). A step is one scan, one exchange of minima and one window update. The magnets are
+// numbered in cell order ("slots"; the cell itself when every cell holds one), and chunk c of 32
+// slots belongs to warp c mod W of the instance's W owner warps: the same lane scans a slot,
+// updates its energies and refreshes its bound for the whole run. So what a warp reads it wrote
+// itself, the energies stay in its SM's L1, and no barrier separates an update from the next scan.
+// Per step: two block barriers and, on a cluster, one cluster barrier.
+//   scan      per slot the bound log u + s from the first Philox word (s = b_low beta rounded down,
+//             kept per slot); a warp queues the slots whose bound does not rule them out
+//   barrier   the block's smallest upper bound; what it rules out leaves the queues, the exact keys
+//             of the rest (a few in the block) are computed
+//   exchange  the CTA's winner goes to every CTA of the cluster; each warp takes the minimum itself
+//   update    the owners of the window's slots; meanwhile one helper warp of rank 0, which owns no
+//             slots, computes the switching time, the counters and the stop rule (neel_finalize),
+//             which the next step needs only at its exchange.
+// A switch whose key is clearly below the limit thr (log of the time left, 1e-3 off) happens for
+// certain and its update does not wait for the time; otherwise the helper decides first.
+// Results are those of the step kernels bit for bit (same keys, same updates).
+// Measured (B200), us per step, cutoff 16a, before (all threads scan and update any cell, the record
+// decided by one thread between two cluster barriers) and now: 64 x 64 uncut on one CTA 15.5 -> 9.6,
+// on 16 CTAs 12.2 -> 4.7; 200 x 111 kagome on two CTAs 20.2 -> 11.9, on 16 13.6 -> 6.1. Bound on one
+// CTA: instructions (IPC 2.3, L1 hit rate 99.6%); on 16: the latency of the chain scan 1,800 cycles,
+// exact key 800, exchange 2,100, update 3,100.
+HS_DEV unsigned ordered_f32(float f) {
+    const unsigned b = __float_as_uint(f);
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+HS_DEV float unordered_f32(unsigned b) { return __uint_as_float(b & 0x80000000u ? b & 0x7fffffffu : ~b); }
+HS_DEV float warp_min_f32(float f) { return unordered_f32(__reduce_min_sync(0xffffffffu, ordered_f32(f))); }
+
+// Lane holding the smallest (key, idx) of the warp (idx < 0: no candidate), or -1.
+HS_DEV int warp_kmin_lane(double key, int idx) {
+    uint64_t k = (uint64_t)__double_as_longlong(key + 0.0);
+    k = k >> 63 ? ~k : k | (1ULL << 63);
+    // every lane takes part in every reduction
+    bool c = idx >= 0;
+    const unsigned hi = c ? (unsigned)(k >> 32) : 0xffffffffu;
+    const unsigned mhi = __reduce_min_sync(0xffffffffu, hi);
+    c = c && hi == mhi;
+    const unsigned lo = c ? (unsigned)k : 0xffffffffu;
+    const unsigned mlo = __reduce_min_sync(0xffffffffu, lo);
+    c = c && lo == mlo;
+    const unsigned id = c ? (unsigned)idx : 0xffffffffu;
+    const unsigned mid = __reduce_min_sync(0xffffffffu, id);
+    c = c && id == mid;
+    return __ffs(__ballot_sync(0xffffffffu, c)) - 1;
+}
+
+// What the owner path reads of the lattice, in registers: through the descriptor in shared memory
+// every field would be loaded again after each store to an array (which might alias it): 64 x 64
+// uncut on one CTA 11.0 -> 9.2 us per step.
+struct NeelOwn {
+    int W, w;            // owner warps of the instance, and this one
+    int M, nch;          // slots, chunks
+    float *s;            // bound per slot
+    const int32_t *list; // occupied cells, or null when the slots are the cells
+    double *E, *Ep;      // null without a dipolar energy (a second channel)
+    int8_t *m;
+    float *mm;
+    const float *zee, *zeep, *EB, *K, *Kpo;
+    double beta, m_perp_factor;
+    int nx, ny, wy, wx, dip_wrap, use_perp, barrier_method;
+    float pref2, inv_W, inv_nx;
+};
+
+HS_DEV int own_cell(const NeelOwn &O, int j) { return O.list ? __ldg(O.list + j) : j; }
+
+// First slot at or after row y.
+HS_DEV int own_row(const HsLattice &L, const NeelOwn &O, const int *rowpre, int y) {
+    if (!O.list) return y * L.nx;
+    if (L.uy <= NEEL_OWN_UY) {
+        const int p = y / L.uy;
+        return p * rowpre[L.uy] + rowpre[y - p * L.uy];
+    }
+    int lo = 0, hi = O.M;                 // a period longer than the table: search the sorted list
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(L.nonzero + mid) < y * L.nx) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// What a cell's bound needs besides its energies and spin.
+struct OwnStatic { float zee, zeep, EB; };
+HS_DEV OwnStatic own_static(const NeelOwn &O, int i, bool v) {
+    return OwnStatic{(v && O.zee) ? __ldg(O.zee + i) : 0.f, (v && O.zee && O.use_perp) ? __ldg(O.zeep + i) : 0.f,
+                     v ? __ldg(O.EB + i) : 0.f};
+}
+// Bound of a cell with energies E, Ep and spin m, rounded down.
+HS_DEV float own_bound(const NeelOwn &O, const OwnStatic &c, double E, double Ep, int m) {
+    if (O.zee) {
+        E += (double)m * (double)c.zee;
+        if (O.use_perp) Ep += (double)m * (double)c.zeep;
+    }
+    double b1, b2;
+    hs_barriers_from(O, E, Ep, (double)c.EB, b1, b2);
+    return __double2float_rd(fmin(b1, b2) * O.beta);
+}
+
+// Exact log-domain key of occupied cell i from its (owned) energies: the operations of
+// neel_scan_range with b_min = 0, so both give the same key bit for bit.
+HS_DEV HsKeyIdx own_key(const NeelOwn &O, int i, uint32_t call_lo, uint32_t call_hi, const HsRoundKeys &RK) {
+    double E = O.E ? O.E[i] : 0.0, Ep = O.Ep ? O.Ep[i] : 0.0;
+    const int mv = O.m[i];
+    const float mm = O.mm[i];
+    const double uk = hs_u53_of(hs_philox_rk((uint32_t)i, call_lo, call_hi, 0u, RK));
+    if (O.zee) { E += (double)mv * (double)__ldg(O.zee + i); if (O.use_perp) Ep += (double)mv * (double)__ldg(O.zeep + i); }
+    double b1, b2;
+    hs_barriers_from(O, E, Ep, (double)__ldg(O.EB + i), b1, b2);
+    const double le1 = (double)hs_log_exp1_f32(uk);
+    double key;
+    if (!O.use_perp) key = le1 + b1 * O.beta;
+    else {
+        const double bm = fmin(b1, b2), dd = fabs(b1 - b2);
+        key = le1 + bm * O.beta - (double)log1pf(expf((float)(-dd * O.beta)));
+    }
+    return HsKeyIdx{key, i, b1, b2, mm, mv};
+}
+
+// The warp's part of a scan: queues the slots that may hold the smallest key and returns an upper
+// bound T of the smallest key among its slots. `best` collects exact keys when the queue fills up.
+template <int OWN_UNR>       // chunks in flight
+HS_DEV float own_scan_u(const NeelOwn &O, uint64_t call, const HsRoundKeys &RK, int *q, float *ql,
+                      int &qn, HsKeyIdx &best) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t call_lo = (uint32_t)call, call_hi = (uint32_t)(call >> 32);
+    const float slack = O.use_perp ? 0.69314722f + 1e-4f : 1e-4f;   // two channels lower a key by at most ln 2
+    float T = INFINITY;   // warp-uniform, as qn
+    qn = 0;
+    auto load = [&](int c, int (&ci)[OWN_UNR], float (&sc)[OWN_UNR]) {
+#pragma unroll
+        for (int k = 0; k < OWN_UNR; ++k) {
+            const int cc = c + k * O.W, j = 32 * cc + lane;
+            const bool v = cc < O.nch && j < O.M;
+            ci[k] = v ? own_cell(O, j) : 0;
+            sc[k] = v ? O.s[j] : INFINITY;
+        }
+    };
+    int ci[OWN_UNR];
+    float sc[OWN_UNR];
+    load(O.w, ci, sc);
+    for (int c = O.w; c < O.nch; c += OWN_UNR * O.W) {
+        int cn[OWN_UNR];
+        float sn[OWN_UNR];
+        load(c + OWN_UNR * O.W, cn, sn);
+        uint32_t x[OWN_UNR];
+#pragma unroll
+        for (int k = 0; k < OWN_UNR; ++k) x[k] = hs_philox_rk((uint32_t)ci[k], call_lo, call_hi, 0u, RK).x;
+        // lower bounds, rounded down; the slot of the lane's smallest gives an upper bound
+        float lb[OWN_UNR], lmin = INFINITY, smin = INFINITY;
+        uint32_t xmin = 0u;
+#pragma unroll
+        for (int k = 0; k < OWN_UNR; ++k) {
+            const float u = (float)(x[k] >> 8) * 5.9604644775390625e-08f;
+            lb[k] = __fadd_rd(__fadd_rd(__logf(u), sc[k]), -slack);
+            if (sc[k] == INFINITY) lb[k] = INFINITY;     // log 0 + inf is not a number
+            if (lb[k] < lmin) { lmin = lb[k]; xmin = x[k]; smin = sc[k]; }
+        }
+        if (__any_sync(0xffffffffu, lmin <= T && lmin < INFINITY)) {
+            // An upper bound of the exact key (own_key): u53 < u24 + 2^-24 and E1 = -log1p(-u) grows
+            // with u, the two-channel term only lowers the key, s is below the next float up;
+            // 1e-4 covers the float logarithms (absolute errors below 1e-5), the sums round up.
+            const float uh = (float)(xmin >> 8) * 5.9604644775390625e-08f + 5.9604644775390625e-08f;
+            const float le = __logf(-log1pf(-uh));
+            const float sh = __fadd_ru(smin, __fmaf_ru(fabsf(smin), 2.4e-7f, 1e-30f));
+            const float ub = lmin < INFINITY ? __fadd_ru(__fadd_ru(le, sh), 1e-4f) : INFINITY;
+            T = fminf(T, warp_min_f32(ub));
+        }
+#pragma unroll
+        for (int k = 0; k < OWN_UNR; ++k) {
+            const bool adm = lb[k] <= T && lb[k] < INFINITY;
+            const unsigned m = __ballot_sync(0xffffffffu, adm);
+            if (!m) continue;
+            const int pos = qn + __popc(m & below);
+            if (adm) { q[pos] = ci[k]; ql[pos] = lb[k]; }
+            qn += __popc(m);
+            if (qn > NEEL_QCAP - 32) {       // full: drop what T rules out by now, else evaluate
+                __syncwarp();
+                int n = 0;
+                for (int b = 0; b < qn; b += 32) {
+                    const bool v = b + lane < qn;
+                    const int i = v ? q[b + lane] : 0;
+                    const float l = v ? ql[b + lane] : INFINITY;
+                    const unsigned keep = __ballot_sync(0xffffffffu, v && l <= T);
+                    __syncwarp();
+                    if (v && l <= T) { q[n + __popc(keep & below)] = i; ql[n + __popc(keep & below)] = l; }
+                    n += __popc(keep);
+                    __syncwarp();
+                }
+                qn = n;
+                if (qn > NEEL_QCAP - 32) {
+                    for (int b = 0; b < qn; b += 32)
+                        if (b + lane < qn) best = hs_kmin(best, own_key(O, q[b + lane], call_lo, call_hi, RK));
+                    T = fminf(T, warp_min_f32(best.idx >= 0 ? __double2float_ru(best.key) : INFINITY));
+                    qn = 0;
+                    __syncwarp();
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < OWN_UNR; ++k) { ci[k] = cn[k]; sc[k] = sn[k]; }
+    }
+    __syncwarp();
+    return T;
+}
+
+HS_DEV float own_scan(const NeelOwn &O, uint64_t call, const HsRoundKeys &RK, int *q, float *ql, int &qn,
+                      HsKeyIdx &best) {
+    // a warp with a single chunk does not pay for empty ones
+    return O.w + O.W >= O.nch ? own_scan_u<1>(O, call, RK, q, ql, qn, best) : own_scan_u<3>(O, call, RK, q, ql, qn, best);
+}
+
+// A switch: its cell, new spin and new moment, its kernels at offset 0.
+struct OwnSwitch { int i0, sy, sx, sm; float smm; const float *K0, *Kp0; };
+
+// Chunks c, c + W, ... < c1 of a window update, slots [j0, j1), U chunks in flight. The arithmetic
+// per cell is that of update_one.
+template <int U>
+HS_DEV void own_update_chunks(const NeelOwn &O, const OwnSwitch &w, int c, int c1, int j0, int j1) {
+    const int lane = threadIdx.x & 31;
+    const int nx = O.nx, ny = O.ny, wy = O.wy, wx = O.wx, KW = 2 * wx + 1;
+    const bool wrap = O.dip_wrap != 0;
+    for (; c < c1; c += U * O.W) {
+        int ci[U], j[U], ko[U];
+        bool in[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            j[k] = 32 * (c + k * O.W) + lane;
+            in[k] = j[k] >= j0 && j[k] < j1;
+            ci[k] = in[k] ? own_cell(O, j[k]) : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            int row = ci[k] < (1 << 24) ? (int)((float)ci[k] * O.inv_nx) : ci[k] / nx;
+            int col = ci[k] - row * nx;
+            if (col < 0) { --row; col += nx; }
+            else if (col >= nx) { ++row; col -= nx; }
+            int dy = row - w.sy, dx = col - w.sx;
+            if (wrap) {
+                dy = dy < 0 ? dy + ny : dy; dy = 2 * dy >= ny ? dy - ny : dy;
+                dx = dx < 0 ? dx + nx : dx; dx = 2 * dx >= nx ? dx - nx : dx;
+            }
+            in[k] = in[k] && dy >= -wy && dy <= wy && dx >= -wx && dx <= wx;
+            ko[k] = dy * KW + dx;
+        }
+        float kv[U], kp[U], mv[U];
+        double ev[U], pv[U];
+        int ms[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int i = ci[k];
+            const bool src = i == w.i0;
+            kv[k] = (in[k] && w.K0) ? __ldg(w.K0 + ko[k]) : 0.f;
+            kp[k] = (in[k] && w.Kp0) ? __ldg(w.Kp0 + ko[k]) : 0.f;
+            mv[k] = in[k] ? (src ? w.smm : O.mm[i]) : 0.f;
+            ms[k] = in[k] ? (src ? w.sm : (int)O.m[i]) : 0;
+            ev[k] = (in[k] && O.E) ? O.E[i] : 0.0;
+            pv[k] = (in[k] && O.Ep) ? O.Ep[i] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            if (!in[k]) continue;
+            const int i = ci[k];
+            const float acc = w.smm * kv[k], accp = w.smm * kp[k];
+            double e = ev[k] + (double)(O.pref2 * (mv[k] * acc));
+            double p = pv[k] + (double)(O.pref2 * (mv[k] * accp));
+            if (i == w.i0) {
+                e = -e; p = -p;
+                O.m[i] = (int8_t)w.sm;
+                O.mm[i] = w.smm;
+            }
+            if (O.E) O.E[i] = e;
+            if (O.Ep) O.Ep[i] = p;
+            O.s[j[k]] = own_bound(O, own_static(O, i, true), e, O.use_perp ? p : 0.0, ms[k]);
+        }
+    }
+}
+
+// Window update of the switch of cell i0 (new moment smm, new spin sm) for the slots this warp owns, with
+// their bounds.
+HS_DEV void own_update(const HsLattice &L, const NeelOwn &O, const int *rowpre, int i0, float smm, int sm) {
+    const int lane = threadIdx.x & 31;
+    const int nx = O.nx, ny = O.ny, wy = O.wy, wx = O.wx;
+    const int sy = i0 / nx, sx = i0 - sy * nx;
+    const bool wrap = O.dip_wrap != 0;
+    const int sub = O.E ? hs_sub(L, sy, sx) : -1;
+    const int64_t k0 = ((int64_t)max(sub, 0) * (2 * wy + 1) + wy) * (2 * wx + 1) + wx;      // offset 0 of the kernel
+    const OwnSwitch w{i0, sy, sx, sm, smm, sub >= 0 ? O.K + k0 : nullptr, (sub >= 0 && O.Ep) ? O.Kpo + k0 : nullptr};
+    // rows [r0, r1) and, wrapped, [q0, q1)
+    int r0 = max(0, sy - wy), r1 = min(ny, sy + wy + 1), q0 = 0, q1 = 0;
+    if (wrap) {
+        if (2 * wy + 1 >= ny) { r0 = 0; r1 = ny; }
+        else if (sy - wy < 0) { q0 = sy - wy + ny; q1 = ny; }
+        else if (sy + wy >= ny) { q0 = 0; q1 = sy + wy + 1 - ny; }
+    }
+    for (int part = 0; part < 2; ++part) {
+        const int y0 = part ? q0 : r0, y1 = part ? q1 : r1;
+        if (y0 >= y1) continue;
+        const int j0 = y0 == 0 ? 0 : own_row(L, O, rowpre, y0), j1 = y1 == ny ? O.M : own_row(L, O, rowpre, y1);
+        const int c0 = j0 >> 5, c1 = (j1 + 31) >> 5;
+        // the warp's first chunk at or after c0
+        int c = (int)((float)c0 * O.inv_W) * O.W + O.w;
+        while (c < c0) c += O.W;
+        while (c - O.W >= c0) c -= O.W;
+        // a warp with a single chunk does not pay for an empty one
+        if (c + O.W >= c1) { if (c < c1) own_update_chunks<1>(O, w, c, c1, j0, j1); }
+        else own_update_chunks<2>(O, w, c, c1, j0, j1);
+    }
+}
+
+// Can the instance's Néel steps run on owned cells?
+HS_DEV bool neel_owned(const HsInstance &I) {
+    return I.L.beta_uniform > 0.0 && !I.L.has_exchange &&
+           I.scratch_bytes >= HS_NEEL_CACHE_OFFSET + 4 * (int64_t)I.L.nx * I.L.ny;
+}
+
+// All Néel steps of an instance on owned cells. `go_next(next)`, on rank 0's helper lane, is whether
+// step `next` runs.
+template <int CS, typename Go>
+HS_DEV void neel_run_owned(EngShared &sh, const RunSync<CS> &S, int rank, int SCS, int64_t budget, Go go_next) {
+    const HsInstance &I = sh.I;
+    const HsLattice &L = sh.I.L;
+    HsCounters *const C = &sh.C;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const bool helper = rank == 0 && warp == nwarps - 1;
+    NeelOwn O;
+    O.W = SCS * nwarps - 1;
+    O.w = rank * nwarps + warp - (rank ? 1 : 0);
+    O.list = (int64_t)L.n_occ < (int64_t)L.nx * L.ny ? L.nonzero : nullptr;
+    O.M = O.list ? L.n_occ : L.nx * L.ny;
+    O.nch = (O.M + 31) >> 5;
+    O.s = reinterpret_cast<float *>(reinterpret_cast<char *>(I.scratch) + HS_NEEL_CACHE_OFFSET);
+    const bool dip = L.has_dipolar != 0, two = L.use_perp != 0;
+    O.E = dip ? L.E_dip : nullptr;
+    O.Ep = dip && two ? L.E_dip_perp : nullptr;
+    O.m = L.m; O.mm = L.mm;
+    O.zee = L.zee; O.zeep = L.zee_perp; O.EB = L.E_B; O.K = L.K; O.Kpo = L.Kpo;
+    O.beta = L.beta_uniform; O.m_perp_factor = L.m_perp_factor;
+    O.nx = L.nx; O.ny = L.ny;
+    O.wy = dip ? L.dip_wy : 0; O.wx = dip ? L.dip_wx : 0; O.dip_wrap = dip ? L.dip_wrap : 0;
+    O.use_perp = L.use_perp; O.barrier_method = L.barrier_method;
+    O.pref2 = (float)(2.0 * L.dip_pref);
+    O.inv_W = 1.0f / (float)O.W;
+    O.inv_nx = 1.0f / (float)O.nx;
+    // occupied cells of a period of uy rows (the first ones of the list)
+    const bool table = O.list && L.uy <= NEEL_OWN_UY;
+    if (table)
+        for (int k = threadIdx.x; k <= L.uy; k += blockDim.x) sh.rowpre[k] = 0;
+    __syncthreads();
+    if (table)
+        for (int k = threadIdx.x; k < min(O.M, L.uy * L.nx); k += blockDim.x) {
+            const int y = __ldg(L.nonzero + k) / L.nx;
+            if (y < L.uy) atomicAdd(&sh.rowpre[y + 1], 1);
+        }
+    __syncthreads();
+    if (table && threadIdx.x == 0)
+        for (int k = 0; k < L.uy; ++k) sh.rowpre[k + 1] += sh.rowpre[k];
+    if (!helper)
+        for (int c = O.w; c < O.nch; c += O.W) {
+            const int j = 32 * c + lane;
+            if (j >= O.M) break;
+            const int i = own_cell(O, j);
+            O.s[j] = own_bound(O, own_static(O, i, true), O.E ? __ldcg(O.E + i) : 0.0, O.Ep ? __ldcg(O.Ep + i) : 0.0, (int)__ldcg(O.m + i));
+        }
+    // helper: whether step `next` runs, and below which key its switch happens for certain
+    const double af = two ? I.attempt_freq / 2.0 : I.attempt_freq;
+    auto publish_next = [&](int64_t next) {
+        int go = 0;
+        double thr = -INFINITY;
+        if (lane == 0) {
+            go = go_next(next);
+            const double left = C->progress ? (C->t_max - (C->t - C->t0)) : C->t_max;
+            if (af > 0.0 && af < INFINITY && left > 0.0) {
+                const double l = log(left) + log(af);
+                thr = left == INFINITY ? INFINITY : l - 1e-3 - 1e-6 * fabs(l);
+            }
+        }
+        go = __shfl_sync(0xffffffffu, go, 0);
+        thr = __shfl_sync(0xffffffffu, thr, 0);
+        S.publish_warp(&sh.go[next & 1], go, SCS);
+        S.publish_warp(&sh.thr[next & 1], thr, SCS);
+    };
+    if (helper) {
+        publish_next(0);
+        S.publish_warp(&sh.call[0], (unsigned long long)C->rng_call, SCS);
+        S.publish_warp(&sh.nsw, C->progress, SCS);
+    }
+    S.all();
+    const uint64_t call0 = sh.call[0];
+    const bool fixed = sh.nsw == 0;          // run(steps): no stop rule but the budget
+    const HsRoundKeys RK = hs_round_keys(L.seed);
+    for (int64_t st = 0;; ++st) {
+        if (fixed && st >= budget) break;
+        const uint64_t call = call0 + (uint64_t)st;
+        const uint32_t call_lo = (uint32_t)call, call_hi = (uint32_t)(call >> 32);
+        HsKeyIdx best{0.0, -1};
+        int qn = 0;
+        float T = INFINITY;
+        if (!helper) T = own_scan(O, call, RK, sh.nq.q[warp], sh.nq.lb[warp], qn, best);
+        if (lane == 0) sh.tw[warp] = T;
+        __syncthreads();
+        T = warp_min_f32(lane < nwarps ? sh.tw[lane] : INFINITY);
+        for (int b = 0; b < qn; b += 32) {
+            const bool v = b + lane < qn && sh.nq.lb[warp][b + lane] <= T;
+            if (__any_sync(0xffffffffu, v) && v) best = hs_kmin(best, own_key(O, sh.nq.q[warp][b + lane], call_lo, call_hi, RK));
+        }
+        {
+            const int wl = __any_sync(0xffffffffu, best.idx >= 0) ? warp_kmin_lane(best.key, best.idx) : -1;
+            if (lane == max(wl, 0)) sh.red[warp] = best;      // idx < 0 when there is none
+        }
+        __syncthreads();
+        const HsKeyIdx *rec = sh.red;
+        int nrec = nwarps;
+        if (CS > 1 && SCS > 1) {
+            if (warp == 0) {
+                const HsKeyIdx r = lane < nwarps ? sh.red[lane] : HsKeyIdx{0.0, -1};
+                const int wl = max(warp_kmin_lane(r.key, r.idx), 0);
+                S.copy_to_all(&sh.part[st & 1][rank], &sh.red[wl], SCS);
+            }
+            S.all();
+            rec = sh.part[st & 1];
+            nrec = SCS;
+        }
+        if (!sh.go[st & 1]) break;
+        const double key = lane < nrec ? rec[lane].key : 0.0;
+        const int wl = warp_kmin_lane(key, lane < nrec ? rec[lane].idx : -1);
+        const HsKeyIdx w = wl >= 0 ? rec[wl] : HsKeyIdx{0.0, -1};
+        const bool certain = wl >= 0 && isfinite(w.key) && w.key < sh.thr[st & 1];
+        bool flip = certain;
+        NeelFlip f{};
+        if (helper && lane == 0) neel_finalize(L, C, sh.I.sw, w, call, 0.0, true, two, I.attempt_freq, &f);
+        if (!certain) {          // uniform over the instance's threads
+            if (helper) S.publish_warp(&sh.n1, (int)__shfl_sync(0xffffffffu, (int)f.flip, 0), SCS);
+            S.all();
+            flip = sh.n1 != 0;
+        }
+        if (helper) {
+            if (lane == 0 && f.flip) {
+                sh.I.sw.y[0] = f.y;
+                sh.I.sw.x[0] = f.x;
+                if (sh.I.sw.mode) sh.I.sw.mode[0] = 0;
+            }
+            publish_next(st + 1);
+        } else if (flip) own_update(L, O, sh.rowpre, w.idx, -w.mm, -w.m);
+    }
+}
 
 // Run instance ii to the end of its step budget (or its stop rule) on the whole cluster
 // (`rank` = this CTA's rank) or, in CTA mode, on this CTA alone (rank 0).
@@ -510,7 +964,7 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
     // to every CTA in slot st & 1; the barriers that end step st - 1 make them visible, so a
     // step needs no barrier of its own for this. Slot st & 1 was last read at the start of
     // step st - 2, before that step's barriers, so the write cannot overtake a read.
-    auto decide_next = [&](int64_t next) {
+    auto go_next = [&](int64_t next) {
         int go;
         if (C->done) go = 0;
         else if (C->progress) {
@@ -518,12 +972,19 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
             else { go = hs_progress_continue(C, L.n_occ); if (!go) { C->done = 1; C->n_sw = 0; } }
         }
         else go = next < I.steps;
-        S.publish(&sh.go[next & 1], go);
+        return go;
+    };
+    auto decide_next = [&](int64_t next) {
+        S.publish(&sh.go[next & 1], go_next(next));
         S.publish(&sh.call[next & 1], (unsigned long long)C->rng_call);
     };
-    if (rank == 0 && threadIdx.x == 0) decide_next(0);
-    S.all();
-    for (int64_t st = 0;; ++st) {
+    const bool owned = scheme == HS_SCHEME_NEEL && neel_owned(I);
+    if (owned) neel_run_owned(sh, S, rank, SCS, I.steps, go_next);
+    else {
+        if (rank == 0 && threadIdx.x == 0) decide_next(0);
+        S.all();
+    }
+    for (int64_t st = 0; !owned; ++st) {
         if (!sh.go[st & 1]) break;
         if (scheme == HS_SCHEME_METROPOLIS) {
             if (rank == 0) {
@@ -554,11 +1015,11 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
                     v = fmin(v, fmin(b1, b2));
                 }
                 v = eng_block_dmin(v, sh.dred);
-                if (threadIdx.x == 0) S.to_rank0(sh.part, rank, HsKeyIdx{v, rank});
+                if (threadIdx.x == 0) S.to_rank0(sh.part[0], rank, HsKeyIdx{v, rank});
                 S.all();
                 if (rank == 0 && threadIdx.x == 0) {
                     double b = INFINITY;
-                    for (int r = 0; r < SCS; ++r) b = fmin(b, sh.part[r].key);
+                    for (int r = 0; r < SCS; ++r) b = fmin(b, sh.part[0][r].key);
                     C->bmin = b;
                     S.publish(&sh.dred[0], b);
                 }
@@ -567,37 +1028,16 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
                 S.all();
             }
             const bool two = L.use_perp != 0;
-            // barrier cache: uniform beta, no exchange (its neighbours change outside the window)
-            float *cache = (unif && !L.has_exchange && I.scratch_bytes >= HS_NEEL_CACHE_OFFSET + 4 * N)
-                               ? reinterpret_cast<float *>(reinterpret_cast<char *>(I.scratch) + HS_NEEL_CACHE_OFFSET)
-                               : nullptr;
-            HsKeyIdx best{0.0, -1};
-            if (cache && st > 0) {
-                // as many whole warps as give every thread a full chunk of cells (all threads
-                // for large lattices): a small lattice is scanned by fewer warps, each with
-                // the same chain of loads and exact evaluations as a full one
-                const int64_t M = 4 * (int64_t)L.n_occ < 3 * N ? (int64_t)L.n_occ : N;
-                const int64_t Pw = min(gs, (M + NEEL_UNR * 32 - 1) / (NEEL_UNR * 32) * 32);
-                if (gt - (threadIdx.x & 31) < Pw) best = neel_scan_cached(L, cache, gt, Pw, N, call, best, sh.nq[warp]);
-            } else {
-                best = neel_scan_range(L, gt, gs, N, call, bmin, best, cache);
-            }
-            best = eng_block_kmin(best, sh.red, cache && st > 0);
-            if (threadIdx.x == 0) S.to_rank0(sh.part, rank, best);
+            HsKeyIdx best = neel_scan_range(L, gt, gs, N, call, bmin, HsKeyIdx{0.0, -1});
+            best = eng_block_kmin(best, sh.red);
+            if (threadIdx.x == 0) S.to_rank0(sh.part[0], rank, best);
             S.all();
             NeelFlip flip{};   // thread 0 of rank 0: the step's flip, written after the handover
             if (rank == 0 && threadIdx.x == 0) {
                 HsKeyIdx w{0.0, -1};
-                for (int r = 0; r < SCS; ++r) w = hs_kmin(w, sh.part[r]);
+                for (int r = 0; r < SCS; ++r) w = hs_kmin(w, sh.part[0][r]);
                 neel_finalize(L, C, sw, w, call, bmin, unif, two, I.attempt_freq, &flip);
                 const int n1 = C->n_sw;
-                if (cache && !L.has_dipolar && n1 > 0) {  // no window update: refresh the flipped cell
-                    const int64_t i = w.idx;
-                    const double m = (double)flip.m_new;
-                    double E = 0.0, Ep = 0.0;
-                    if (L.zee) { E = m * (double)L.zee[i]; if (two) Ep = m * (double)L.zee_perp[i]; }
-                    cache[i] = neel_cache_value(L, E, Ep, (double)L.E_B[i]);
-                }
                 // hand the switch to every CTA through shared memory (no global round trip)
                 S.publish(&sh.n1, n1);
                 if (n1 > 0) {
@@ -614,7 +1054,7 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
             // and the writes are ordered before the next step by the barrier that ends this one.
             S.all_then(rank == 0 && threadIdx.x == 0 && flip.flip, [&] { neel_apply(L, sw, flip); });
             if (L.has_dipolar && sh.n1 > 0)
-                update_one(L, sh.y1, sh.x1, sh.mm1, (int8_t)sh.m1, rank * blockDim.x + threadIdx.x, SCS * blockDim.x, cache);
+                update_one(L, sh.y1, sh.x1, sh.mm1, rank * blockDim.x + threadIdx.x, SCS * blockDim.x);
             S.all();
         } else {  // Wolff
             if (rank == 0) {

@@ -1145,9 +1145,11 @@ HS_HD inline void hs_metro_sizes(const HsLattice &L, const HsGridPlan &P, int &c
 
 // Barriers of hotspice/core.py:625-656 from an already-loaded total energy E, perpendicular
 // energy Ep (before m_perp_factor) and E_B.
-HS_DEV void hs_barriers_from(const HsLattice &L, double E, double Ep, double EB, double &b1, double &b2) {
+// (V: HsLattice, or a copy of its fields use_perp, barrier_method and m_perp_factor.)
+template <typename V>
+HS_DEV void hs_barriers_from(const V &L, double E, double Ep, double EB, double &b1, double &b2) {
     const double dE = -2.0 * E;
-    const double Ecur = -dE / 2.0;
+    const double Ecur = E;             // -dE / 2, exactly
     if (!L.use_perp) {
         double b;
         if (L.barrier_method == HS_BARRIER_SIMPLE) {
@@ -1175,22 +1177,16 @@ HS_DEV void hs_barriers_from(const HsLattice &L, double E, double Ep, double EB,
 // for the fast logarithm) is a lower bound of the key. The (key, index) minimum does not depend
 // on the visiting order or on the skipping (ties go to the smaller index; only cells whose key
 // is strictly larger than a key already seen are skipped).
-// Néel barrier cache (engine only): per cell s = b_low * beta (uniform beta), rounded down to
-// float, +inf for an empty cell. It lives in the Néel scratch at this offset and is valid only
-// inside one engine launch (built by the launch's first step, refreshed by the window update).
+// Bounds of the engine's Néel path: per magnet s = b_low * beta (uniform beta), rounded down to
+// float. They live in the Néel scratch at this offset and are valid only inside one engine launch
+// (built at an instance's start, refreshed by the window update).
 constexpr int64_t HS_NEEL_CACHE_OFFSET = 65536;
-HS_DEV float neel_cache_value(const HsLattice &L, double E, double Ep, double EB) {
-    double b1, b2;
-    hs_barriers_from(L, E, Ep, EB, b1, b2);
-    return __double2float_rd(fmin(b1, b2) * L.beta_uniform);
-}
-
 #ifndef HS_NEEL_UNROLL
 #define HS_NEEL_UNROLL 3
 #endif
 constexpr int NEEL_UNR = HS_NEEL_UNROLL;
 HS_DEV HsKeyIdx neel_scan_range(const HsLattice &L, int64_t start64, int64_t stride64, int64_t N64, uint64_t call,
-                                double bmin, HsKeyIdx best, float *cache = nullptr) {
+                                double bmin, HsKeyIdx best) {
     const bool two = L.use_perp != 0;
     const bool sparse = 4 * (int64_t)L.n_occ < 3 * N64;
     const int M = sparse ? L.n_occ : (int)N64;     // cell indices fit in int (HsKeyIdx.idx)
@@ -1238,7 +1234,6 @@ HS_DEV HsKeyIdx neel_scan_range(const HsLattice &L, int64_t start64, int64_t str
             btv[k] = L.beta_uniform > 0.0 ? L.beta_uniform : (double)bt[k];
             const double bm = two ? fmin(b1v[k], b2v[k]) : b1v[k];
             lb[k] = (double)__logf((float)u[k]) + (bm - bmin) * btv[k] - slack;
-            if (cache && base + k * stride < M) cache[ci[k]] = oc[k] ? __double2float_rd(bm * btv[k]) : INFINITY;
         }
 #pragma unroll
         for (int k = 0; k < NEEL_UNR; ++k) {
@@ -1258,133 +1253,5 @@ HS_DEV HsKeyIdx neel_scan_range(const HsLattice &L, int64_t start64, int64_t str
     return best;
 }
 
-// Exact log-domain key of occupied cell i from its energies (uniform beta, b_min = 0): the
-// operations of neel_scan_range, so both give the same key bit for bit.
-HS_DEV HsKeyIdx neel_key_exact(const HsLattice &L, int i, uint32_t call_lo, uint32_t call_hi, const HsRoundKeys &RK) {
-    const bool two = L.use_perp != 0;
-    const double beta = L.beta_uniform;
-    const double uk = hs_u53_of(hs_philox_rk((uint32_t)i, call_lo, call_hi, 0u, RK));
-    double E = L.has_dipolar ? __ldcg(L.E_dip + i) : 0.0;
-    double Ep = (L.has_dipolar && two) ? __ldcg(L.E_dip_perp + i) : 0.0;
-    const int mv = __ldcg(L.m + i);
-    const float mm = __ldcg(L.mm + i);   // carried to the decision (same round trip)
-    if (L.zee) { E += (double)mv * (double)__ldg(L.zee + i); if (two) Ep += (double)mv * (double)__ldg(L.zee_perp + i); }
-    double b1, b2;
-    hs_barriers_from(L, E, Ep, (double)__ldg(L.E_B + i), b1, b2);
-    const double le1 = (double)hs_log_exp1_f32(uk);
-    double key;
-    if (!two) key = le1 + b1 * beta;
-    else {
-        const double bm = fmin(b1, b2), dd = fabs(b1 - b2);
-        key = le1 + bm * beta - (double)log1pf(expf((float)(-dd * beta)));
-    }
-    return HsKeyIdx{key, i, b1, b2, mm, mv};
-}
-
-// Per-warp queue of the cached scan (shared memory, ints): cells whose lower bound does not rule
-// them out wait there and are evaluated 32 at a time, one per lane.
+// Per-warp queue of the engine's scan (shared memory): slots whose lower bound does not rule them out.
 constexpr int NEEL_QCAP = 64;
-
-// An upper bound of the exact key of a cell (neel_key_exact) from its first Philox word and its
-// cached s = b_low beta rounded down: u53 < u24 + 2^-24 and E1 = -log1p(-u) grows with u, the
-// two-channel term only lowers the key, s is below the next float up; 1e-4 covers the float
-// rounding of the logarithms (their absolute errors here are below 1e-5).
-HS_DEV double neel_key_upper(HsU4 w, float s) {
-    const float uh = hs_u24_low(w) + 5.9604644775390625e-08f;   // exact: a multiple of 2^-24 <= 1
-    const float le = __logf(-log1pf(-uh));
-    const double sh = (double)s + fabs((double)s) * 2.4e-7 + 1e-30;
-    return (double)le + sh + 1e-4;
-}
-
-// The same scan from the barrier cache (uniform beta, b_min = 0): per cell the cached
-// s = b_low beta, the Philox variate and the lower bound log u + s; the exact key (computed as
-// in neel_scan_range, from the energies) only for the cells the bound does not rule out.
-// Warp-collective: the 32 lanes of a warp call it together with consecutive `start`s
-// (start = warp base + lane). The warp keeps T, an upper bound of the smallest key among the
-// cells it has seen (the minimum of the cells' upper bounds, neel_key_upper, and of the exact
-// keys found), and admits a cell only when its lower bound is not above T. Admitted cells go to
-// the warp's queue `q` (NEEL_QCAP ints) in ballot order and are evaluated exactly when 32 or
-// more wait, with every lane busy: a per-lane branch to the exact evaluation would cost the warp
-// that evaluation on almost every cell, since some lane of 32 usually admits one. The cell of
-// the smallest key always has its lower bound below T (every upper bound is at least that key),
-// so every cell that can win or tie is evaluated, and the (key, index) minimum is that of the
-// exhaustive scan. Returns the warp's minimum on every lane.
-HS_DEV HsKeyIdx neel_scan_cached(const HsLattice &L, const float *cache, int64_t start64, int64_t stride64, int64_t N64,
-                                 uint64_t call, HsKeyIdx best, int *q) {
-    const bool two = L.use_perp != 0;
-    const bool sparse = 4 * (int64_t)L.n_occ < 3 * N64;
-    const int M = sparse ? L.n_occ : (int)N64;
-    const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    const int start0 = (int)start64 - lane, stride = (int)stride64;
-    const double slack = (two ? 0.6931471805599453 : 0.0) + 1e-4;
-    const HsRoundKeys RK = hs_round_keys(L.seed);
-    const uint32_t call_lo = (uint32_t)call, call_hi = (uint32_t)(call >> 32);
-    if (__any_sync(0xffffffffu, best.idx >= 0)) best = hs_warp_kmin(best);
-    double T = best.idx >= 0 ? best.key : INFINITY;   // warp-uniform
-    int qn = 0;                                       // warp-uniform
-    auto flush = [&]() {
-        __syncwarp();
-        for (int b = 0; b < qn; b += 32) {
-            HsKeyIdx c{0.0, -1};
-            if (b + lane < qn) c = neel_key_exact(L, q[b + lane], call_lo, call_hi, RK);
-            best = hs_kmin(best, hs_warp_kmin(c));
-        }
-        if (best.idx >= 0) T = fmin(T, best.key);
-        qn = 0;
-        __syncwarp();
-    };
-    // cell indices and cached bounds of the chunk at `base` (cells beyond M: index 0, bound +inf)
-    auto load = [&](int base, int *c, float *b) {
-#pragma unroll
-        for (int k = 0; k < NEEL_UNR; ++k) {
-            const int j = base + lane + k * stride;
-            c[k] = j < M ? (sparse ? __ldg(L.nonzero + j) : j) : 0;
-        }
-#pragma unroll
-        for (int k = 0; k < NEEL_UNR; ++k) b[k] = base + lane + k * stride < M ? __ldcg(cache + c[k]) : INFINITY;
-    };
-    int ci[NEEL_UNR];
-    float sc[NEEL_UNR];
-    load(start0, ci, sc);
-    for (int base = start0; base < M; base += stride * NEEL_UNR) {   // warp-uniform trip count
-        // the next chunk's loads are issued first and complete while this chunk computes
-        int cn[NEEL_UNR];
-        float sn[NEEL_UNR];
-        load(base + stride * NEEL_UNR, cn, sn);
-        HsU4 wv[NEEL_UNR];
-#pragma unroll
-        for (int k = 0; k < NEEL_UNR; ++k) wv[k] = hs_philox_rk((uint32_t)ci[k], call_lo, call_hi, 0u, RK);
-        // bounds from the first Philox word (below u53): the FP64 variate only for admitted cells
-        double lbk[NEEL_UNR];
-        double lmin = INFINITY;   // the lane's smallest bound of the chunk, with its word and s
-        HsU4 wmin = wv[0];
-        float smin = sc[0];
-#pragma unroll
-        for (int k = 0; k < NEEL_UNR; ++k) {
-            lbk[k] = sc[k] != INFINITY ? (double)__logf(hs_u24_low(wv[k])) + (double)sc[k] - slack : INFINITY;
-            if (lbk[k] < lmin) { lmin = lbk[k]; wmin = wv[k]; smin = sc[k]; }
-        }
-        if (__any_sync(0xffffffffu, lmin <= T)) {
-            // lower T with the upper bound of each lane's best cell of the chunk (warp-uniform)
-            double t = lmin <= T ? fmin(T, neel_key_upper(wmin, smin)) : T;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t = fmin(t, __shfl_xor_sync(0xffffffffu, t, o));
-            T = t;
-        }
-#pragma unroll
-        for (int k = 0; k < NEEL_UNR; ++k) {
-            const bool adm = sc[k] != INFINITY && lbk[k] <= T;
-            const unsigned m = __ballot_sync(0xffffffffu, adm);
-            if (m) {
-                if (adm) q[qn + __popc(m & below)] = ci[k];
-                qn += __popc(m);
-                if (qn >= 32) flush();
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < NEEL_UNR; ++k) { ci[k] = cn[k]; sc[k] = sn[k]; }
-    }
-    if (qn) flush();
-    return best;
-}

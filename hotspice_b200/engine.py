@@ -51,21 +51,21 @@ def _bind():
 
 def step_model(mm: Magnets) -> tuple[float, float, float]:
     """Device time of one step as (fixed us, cell-dependent us on one CTA, exponent alpha): on a
-    cluster of cs CTAs a step takes fixed + part / cs**alpha. Calibrated on B200 with single
-    instances of the bench lattices (n = 32..512, cluster sizes 1, 4, 16): the cell-dependent
-    part grows like c N^beta with the lattice's occupancy class (dense / half / sparse, which
-    also carries the perpendicular channel of the in-plane lattices), Néel scans spread over the
-    cluster like cs^0.62 and Metropolis steps like cs^0.5; a Wolff step grows its cluster on one
-    CTA and costs 10-17 us above the critical temperature. Inside a full batch the model ranks
-    runs less well (it underestimates how much two CTAs speed up a large Néel scan), so a
-    batch's launch plan is best measured (:meth:`BatchEngine.tune_split`)."""
+    cluster of cs CTAs a step takes fixed + part / cs**alpha, and on more than one CTA the exchange
+    (:func:`model_time`). Calibrated on B200 with single instances of the bench lattices (n = 32..512,
+    cluster sizes 1 to 16): the cell-dependent part grows like c N^beta with the lattice's occupancy
+    class (dense / half / sparse, which also carries the perpendicular channel of the in-plane
+    lattices), Néel steps spread over the cluster like cs^0.85 (512 x 512 dense: 172 us on one CTA,
+    16.5 us on 16; 64 x 64: 7.4 and 5.1 us) and Metropolis steps like cs^0.5; a Wolff step grows its
+    cluster on one CTA and costs 10-17 us above the critical temperature. Inside a full batch the
+    CTAs share the L2, so a batch's launch plan is best measured (:meth:`BatchEngine.tune_split`)."""
     n = mm.nx * mm.ny
     f = mm.n / max(n, 1)
     cls = 0 if f >= 0.75 else (1 if f >= 0.45 else 2)
     sch = mm.params.UPDATE_SCHEME
     if sch == Scheme.NEEL:
-        c, beta = ((0.0116, 0.786), (0.0198, 0.716), (0.0431, 0.646))[cls]
-        return 9.0, c * n ** beta, 0.62
+        c, beta = ((0.00184, 0.915), (0.0040, 0.807), (0.0111, 0.704))[cls]
+        return 4.0, c * n ** beta, 0.85
     if sch == Scheme.WOLFF:
         return 11.0 + 6e-6 * n, 0.0, 0.0
     c, beta = ((0.0037, 0.70), (0.0068, 0.70), (0.0061, 0.73))[cls]
@@ -73,9 +73,10 @@ def step_model(mm: Magnets) -> tuple[float, float, float]:
 
 
 def model_time(m, cs):
-    """Step time (us) of a step model (fixed us, cell-dependent us, alpha) on ``cs`` CTAs."""
+    """Step time (us) of a step model (fixed us, cell-dependent us, alpha) on ``cs`` CTAs; the
+    exchange between the CTAs of a cluster costs about 0.9 us."""
     s0, p, alpha = m
-    return s0 + (p / cs ** alpha if alpha > 0 else p) + 0.1 * (cs - 1)
+    return s0 + (p / cs ** alpha if alpha > 0 else p) + (0.9 if cs > 1 else 0.0) + 0.02 * (cs - 1)
 
 
 def step_time(mm: Magnets, cs: int = 1) -> float:
@@ -89,8 +90,11 @@ def step_cost(mm: Magnets) -> float:
 
 
 def cluster_size_for(mm: Magnets) -> int:
-    """Cluster size for an instance run alone: double the CTAs while that cuts the modelled
-    step time by at least 25%."""
+    """Cluster size for an instance run alone. Néel steps: the fastest by the model (a lone
+    instance has the GPU to itself). Others: double the CTAs while that cuts the modelled step time
+    by at least 25%."""
+    if mm.params.UPDATE_SCHEME == Scheme.NEEL:
+        return min(CLUSTER_SIZES, key=lambda c: (step_time(mm, c), c))
     cs = 1
     while cs < 16 and step_time(mm, 2 * cs) < 0.75 * step_time(mm, cs):
         cs *= 2
