@@ -15,6 +15,7 @@ LIB_PATH = os.path.join(HERE, 'libhotspice_sm100.so')
 
 HS_OK, HS_EINVAL, HS_ENOMEM, HS_ETIMEDOUT, HS_ECUDA, HS_ERANGE = 0, -1, -2, -3, -4, -5
 HS_ST_SELECT_RETRY, HS_ST_SWITCH_OVERFLOW, HS_ST_POISSON_OVERFLOW, HS_ST_WOLFF_OVERFLOW, HS_ST_STEP_CAP = 1, 2, 4, 8, 16
+HS_ST_TIMEOUT = 32
 HS_PROGRESS_STEPS_MAX = 1 << 22
 HS_ENGINE_WS_DEFAULT, HS_ENGINE_WS_MAX = 64 * 1024, 160 * 1024
 HS_SAMPLE_SINGLE, HS_SAMPLE_GRID, HS_SAMPLE_POISSON = 0, 1, 2
@@ -103,6 +104,7 @@ SIGNATURES = {
     'hs_minimize_all': (C.c_int, [C.POINTER(HsLattice), P, C.POINTER(HsSwitchList), C.c_int32, C.c_int32, P,
                                   C.c_int64, P]),
     'hs_relax_check': (C.c_int, [C.POINTER(HsLattice), P, C.c_int32, P, C.c_int64, P]),
+    'hs_relax_run': (C.c_int, [C.POINTER(HsLattice), P, C.c_int32, C.c_int32, C.c_int32, P, C.c_int64, P]),
     'hs_minimize_begin': (C.c_int, [C.POINTER(HsLattice), P, C.c_int64, P]),
     'hs_minimize_step': (C.c_int, [C.POINTER(HsLattice), P, C.POINTER(HsSwitchList), C.c_double, P, C.c_int64, P]),
     'hs_zeeman_set': (C.c_int, [C.c_int64, C.c_int32, P, P, P, C.c_double, C.c_double, P, P, P, P, P]),

@@ -1213,8 +1213,9 @@ class Magnets(ABC):
     def relax(self, verbose=False, **kwargs):
         """hotspice/core.py:827-861: _minimize_all sweeps until one switches nothing, the state
         equals the one two sweeps before, or int(sqrt(nx^2 + ny^2)) sweeps were made. The
-        sweeps and the stop rule run on the device (``EngineConfig.graph_steps`` sweeps per
-        CUDA-graph replay, one host check per replay). Returns nothing, like the reference;
+        sweeps and the stop rule run on the device (hs_relax_run, one host check per 256 sweeps;
+        with ``_simultaneous`` ``EngineConfig.graph_steps`` sweeps per CUDA-graph replay). Returns
+        nothing, like the reference;
         the number of sweeps is kept in ``self.relax_sweeps``."""
         ignore_barrier = bool(kwargs.pop('ignore_barrier', True))
         simultaneous = bool(kwargs.pop('_simultaneous', False))
@@ -1239,10 +1240,19 @@ class Magnets(ABC):
                                                buf.numel(), stream), 'hs_minimize_all')
                 _lib.check(lib.hs_relax_check(L, C, n_max, buf.data_ptr(), buf.numel(), stream), 'hs_relax_check')
         key = ('relax', ignore_barrier, simultaneous, K, buf.data_ptr(), s.y, self._version)
-        for _ in range((n_max + K - 1) // K):
-            self._replay(key, sweeps)
+        made = 0
+        while made < n_max:
+            if simultaneous:
+                self._replay(key, sweeps)
+                made += K
+            else:      # one launch for many sweeps, bounded in length
+                _lib.check(lib.hs_relax_run(L, C, int(ignore_barrier), n_max, 256, buf.data_ptr(), buf.numel(), st),
+                           'hs_relax_run')
+                made += 256
             if self._relax_word(buf, 0):
                 break
+        if self.status & _lib.HS_ST_TIMEOUT:
+            raise RuntimeError(f'device step reported status {self.status} (HS_ST_* bits)')
         self.relax_sweeps = self._relax_word(buf, 1)
         if verbose:
             print(f"Used {self.relax_sweeps} (out of {n_max}) steps in relax().")

@@ -281,6 +281,14 @@ int hs_relax_check(const HsLattice *L, HsCounters *C, int32_t n_max, void *scrat
     return hs_relax_check_impl(*L, C, n_max, scratch, scratch_bytes, (cudaStream_t)stream);
 }
 
+int hs_relax_run(const HsLattice *L, HsCounters *C, int32_t ignore_barrier, int32_t n_max, int32_t max_sweeps,
+                 void *scratch, int64_t scratch_bytes, void *stream) {
+    int rc = check_lattice(L, "hs_relax_run");
+    if (rc) return rc;
+    if (!C || !scratch || n_max < 1 || max_sweeps < 1) { hs_set_error("hs_relax_run: bad argument"); return HS_EINVAL; }
+    return hs_relax_run_impl(*L, C, ignore_barrier, n_max, max_sweeps, scratch, scratch_bytes, (cudaStream_t)stream);
+}
+
 int hs_minimize_begin(const HsLattice *L, void *scratch, int64_t scratch_bytes, void *stream) {
     int rc = check_lattice(L, "hs_minimize_begin");
     if (rc) return rc;

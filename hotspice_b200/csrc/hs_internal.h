@@ -47,6 +47,8 @@ int hs_relax_permute_impl(const HsLattice &L, HsCounters *C, int simultaneous, v
 int hs_relax_subset_impl(const HsLattice &L, HsCounters *C, const HsSwitchList &sw, int i, int ignore_barrier,
                          int simultaneous, void *scratch, int64_t bytes, cudaStream_t st);
 int hs_relax_check_impl(const HsLattice &L, HsCounters *C, int n_max, void *scratch, int64_t bytes, cudaStream_t st);
+int hs_relax_run_impl(const HsLattice &L, HsCounters *C, int ignore_barrier, int n_max, int max_sweeps, void *scratch,
+                      int64_t bytes, cudaStream_t st);
 int hs_minimize_begin_impl(const HsLattice &L, void *scratch, int64_t bytes, cudaStream_t st);
 int hs_minimize_step_impl(const HsLattice &L, HsCounters *C, const HsSwitchList &sw, double frac, void *scratch,
                           int64_t bytes, cudaStream_t st);

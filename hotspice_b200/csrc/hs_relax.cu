@@ -18,7 +18,9 @@
 // two sweeps before, or int(sqrt(nx^2 + ny^2)) sweeps (relax_compare_kernel, relax_end_kernel).
 // Every kernel reads the control state from device memory and returns at once when the stop
 // rule has fired, so the host can enqueue (or replay as a CUDA graph) several sweeps and look
-// at the state once.
+// at the state once. relax() itself runs its sweeps in one cooperative launch instead
+// (relax_grid_kernel): most subgrids of most sweeps switch a handful of magnets, and three
+// launches each were almost all of their time.
 //
 // minimize() (sequential): per iteration the switch energy of every cell, the number n of
 // magnets gaining more than kBT and the first argmin. If n > 0, ceil(0.3 n) of those n switch:
@@ -27,6 +29,7 @@
 // else the argmin switches if it lowers the energy and was not picked three times.
 #include "hs_common.cuh"
 #include "hs_internal.h"
+#include "hs_steps.cuh"
 
 namespace {
 
@@ -251,6 +254,438 @@ __global__ void relax_end_kernel(const HsCounters *C, RelaxBufs B, int n_max) {
     else if (!s->differs) s->done = 1;                 // 2-cycle
     else if (n >= n_max) s->done = 1;
     s->differs = 0;
+}
+
+// ---------------------------------------------------------------------------------------
+// relax(): sweeps and stop rule in one cooperative launch
+// ---------------------------------------------------------------------------------------
+// The lattice is cut into tiles of TY rows x 32 sx columns, so that a row of a tile holds one
+// 32-bit word of candidates of any subgrid; CTA b owns tiles b, b + grid, ... for the whole launch.
+// Per subgrid:
+//   decide   the owners' candidates, a ballot per word into the subgrid's bitmap, and the flips
+//   barrier  with the number of switches (one grid barrier; with an exchange energy another one between decisions and flips,
+//            since a decision may read a neighbour in another tile)
+//   update   every cell of a tile with a switch in reach gathers their contributions straight
+//            from the bitmap, rows and columns ascending: the order of the switch list, hence the
+//            sums of dip_update_kernel bit for bit
+// A subgrid without a switch costs one barrier, and bitmaps alternate, so no barrier separates a
+// subgrid's update from the next one's decisions.
+// Measured on B200: 512 x 512 pinwheel, cutoff 8.3a, about 190 sweeps: 59 ms (launched kernel by
+// kernel) -> 14.5 ms. Bound: three quarters of the subgrids switch at most 20 magnets and take 11 K
+// cycles, decisions 2.1 K, barrier 6 K (half of it waiting for the tile that holds a switch),
+// update 2.5 K.
+struct RelaxGrid {          // zeroed before every launch
+    // grid barriers alternate between two words: arrivals in the low half, the sum of what the CTAs
+    // brought along in the high half
+    unsigned long long bar[2];
+    int abort;              // a barrier gave up
+};
+
+struct RelaxPlan {
+    int sx, sy, TX, TY, tiles_x, tiles, words, rows;   // words per bitmap row, rows of the largest subgrid
+    int ignore_barrier, n_max, max_sweeps;
+    unsigned long long wait_ns;
+    unsigned *bits;         // [2][rows][words]
+    RelaxGrid *g;
+};
+
+constexpr unsigned long long RX_WAIT_NS = 4000000000ULL;   // a grid barrier gives up after 4 s
+
+// Grid barrier number `k` (0, 1, ...) of this launch, adding up every CTA's `v`: the sum of this
+// barrier's, or -1 when it gave up (then on every CTA, sooner or later). `seen` keeps the two words'
+// earlier sums. A CTA still polling a word never meets later arrivals: those of barrier k + 1 go to
+// the other word, and those of k + 2 wait for it at k + 1.
+HS_DEV int grid_barrier(RelaxGrid *g, unsigned k, unsigned v, unsigned (&seen)[2], unsigned long long limit_ns) {
+    __shared__ int s_sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long *word = &g->bar[k & 1];
+        // release: the CTA's writes before the __syncthreads above come before the arrival
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(((unsigned long long)v << 32) | 1ull) : "memory");
+        const unsigned want = ((k >> 1) + 1) * gridDim.x;
+        const unsigned long long t0 = hs_globaltimer_ns();
+        int sum = -1;
+        for (unsigned it = 0;; ++it) {
+            unsigned long long w;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(word) : "memory");
+            if ((unsigned)w >= want) { sum = (int)((unsigned)(w >> 32) - seen[k & 1]); break; }
+            if ((it & 255) == 255) {
+                if (*(volatile int *)&g->abort) break;
+                if (hs_globaltimer_ns() - t0 > limit_ns) { atomicExch(&g->abort, 1); break; }
+            }
+        }
+        s_sum = sum;
+    }
+    __syncthreads();
+    const int sum = s_sum;
+    seen[k & 1] += (unsigned)sum;
+    return sum;
+}
+
+// Cells a..b (inclusive) of an axis within `h` of coordinate v, ascending: one range, or two where
+// they wrap.
+struct Reach { int a[2], b[2], n; };
+HS_DEV Reach reach_of(int v0, int v1, int h, bool wrap, int n) {
+    Reach r;
+    r.n = 1;
+    if (!wrap) { r.a[0] = max(0, v0 - h); r.b[0] = min(n - 1, v1 + h); }
+    else if (v1 - v0 + 2 * h + 1 >= n) { r.a[0] = 0; r.b[0] = n - 1; }
+    else if (v0 - h < 0) { r.a[0] = 0; r.b[0] = v1 + h; r.a[1] = v0 - h + n; r.b[1] = n - 1; r.n = 2; }
+    else if (v1 + h >= n) { r.a[0] = 0; r.b[0] = v1 + h - n; r.a[1] = v0 - h; r.b[1] = n - 1; r.n = 2; }
+    else { r.a[0] = v0 - h; r.b[0] = v1 + h; }
+    return r;
+}
+// Subgrid indices k (coordinate o + k s) in [a, b]: first and one past the last.
+HS_DEV int first_at(int a, int o, int s) { return a <= o ? 0 : (a - o + s - 1) / s; }
+HS_DEV int past_at(int b, int o, int s) { return b < o ? 0 : (b - o) / s + 1; }
+
+struct SubUpdate {
+    int y0, x0, sub, hy, hx, kind;      // kind 0: plain window, 1: minimum image, 2: hs_contrib (truncated, periodic)
+    bool wrap, flip_perp;
+    int mode;
+    const unsigned *bits;
+};
+
+// The candidates in reach of a tile, staged row by row: rows [r0[p], r0[p] + nr[p]) of the subgrid,
+// words [w0[q], w0[q] + nw[q]) of each, in ascending order.
+constexpr int RX_WORDS = 512;            // staged bitmap words (and 32 times as many moments)
+struct RelaxTile {
+    Reach ry, rx;
+    int r0[2], nr[2], w0[2], nw[2], rows, words;
+    HS_DEV int row(int p, int r) const { return (p ? nr[0] : 0) + r - r0[p]; }
+    HS_DEV int word(int q, int w) const { return (q ? nw[0] : 0) + w - w0[q]; }
+};
+constexpr int RX_LIST = 64;              // up to so many switches in reach of a tile go through a list
+struct RelaxHit { int y, x; float mm; };
+struct RelaxShared {
+    unsigned bits[RX_WORDS];
+    float mm[32 * RX_WORDS];             // moments of the staged candidates that switched
+    RelaxHit hit[RX_LIST];
+    int n;                               // switches in reach of the tile
+};
+
+// A warp's 32 columns x RX_V rows of a tile: their energies with the contributions of the switches in
+// reach, in list order. The warp takes one switch at a time, so that a kernel row is read by
+// consecutive lanes (with each lane on its own switches a crowded subgrid's update took 128 K
+// cycles, now 96 K).
+constexpr int RX_V = 8;
+template <bool PERIODIC_CROP>      // kind 2
+HS_DEV void relax_update_warp(const HsLattice &L, const RelaxPlan &P, const SubUpdate &u, const RelaxTile &T,
+                              const RelaxShared &S, bool staged, int y, int x_base, int y_end, int x_end) {
+    const int x = x_base + (threadIdx.x & 31);
+    const int nyv = min(RX_V, y_end - y), nxw = min(32, x_end - x_base);
+    const bool inx = x < x_end;
+    float acc[RX_V] = {}, accp[RX_V] = {};
+    unsigned touched = 0u, neg = 0u;     // bit v: row y + v
+    const int KW = 2 * L.dip_wx + 1;
+    const int64_t k0 = ((int64_t)max(u.sub, 0) * (2 * L.dip_wy + 1) + L.dip_wy) * KW + L.dip_wx;
+    const float *K = L.K + k0, *Kp = L.use_perp ? L.Kpo + k0 : nullptr;
+    const int kind = u.kind, hy = u.hy, hx = u.hx, nx = L.nx, ny = L.ny;
+    const bool has = u.sub >= 0, two = has && Kp;
+    auto apply = [&](int ys, int xs, float ms) {     // warp-uniform arguments
+        if constexpr (PERIODIC_CROP) {
+            if (!inx || !hs_axis_overlap(xs, hx, u.wrap, nx, x, 1)) return;
+#pragma unroll
+            for (int v = 0; v < RX_V; ++v) {
+                if (v >= nyv || !hs_axis_overlap(ys, hy, u.wrap, ny, y + v, 1)) continue;
+                touched |= 1u << v;
+                if (ys == y + v && xs == x) neg |= 1u << v;
+                if (has) hs_contrib(L, SwInfo{ys, xs, u.mode, u.sub, ms}, y + v, x, acc[v], accp[v]);
+            }
+            return;
+        }
+        else {
+        int dx = x - xs;
+        const bool own = dx == 0;
+        if (kind == 1) dx = hs_minimage(dx, nx);
+        const bool in = inx && dx >= -hx && dx <= hx;
+        const float *Kx = K + dx, *Kpx = Kp + dx;
+        float kv[RX_V], kp[RX_V];
+#pragma unroll
+        for (int v = 0; v < RX_V; ++v) {
+            int dy = y + v - ys;
+            if (own && dy == 0) neg |= 1u << v;
+            if (kind == 1) dy = hs_minimage(dy, ny);
+            const bool t = in && v < nyv && dy >= -hy && dy <= hy;
+            if (t) touched |= 1u << v;
+            kv[v] = t && has ? __ldg(Kx + dy * KW) : 0.f;
+            kp[v] = t && two ? __ldg(Kpx + dy * KW) : 0.f;
+        }
+#pragma unroll
+        for (int v = 0; v < RX_V; ++v) { acc[v] += ms * kv[v]; accp[v] += ms * kp[v]; }
+        }
+    };
+    if (staged && S.n <= RX_LIST) {
+        for (int h = 0; h < S.n; ++h) {
+            const RelaxHit hit = S.hit[h];
+            // does its window meet the warp's cells at all?
+            if (!hs_axis_overlap(hit.y, hy, u.wrap, ny, y, nyv) || !hs_axis_overlap(hit.x, hx, u.wrap, nx, x_base, nxw)) continue;
+            apply(hit.y, hit.x, hit.mm);
+        }
+    } else {
+        const Reach ry = reach_of(y, y + nyv - 1, hy, u.wrap, ny), rx = reach_of(x_base, x_base + nxw - 1, hx, u.wrap, nx);
+        int ca[2], cb[2];
+        for (int q = 0; q < rx.n; ++q) { ca[q] = first_at(rx.a[q], u.x0, P.sx); cb[q] = past_at(rx.b[q], u.x0, P.sx); }
+        for (int p = 0; p < ry.n; ++p) {
+            const int r1 = past_at(ry.b[p], u.y0, P.sy);
+            for (int r = first_at(ry.a[p], u.y0, P.sy); r < r1; ++r) {
+                const int ys = u.y0 + r * P.sy;
+                // the row's place in the tile's staging (a warp's range may lie in the tile's other one)
+                const int tp = T.ry.n == 2 && r >= T.r0[1] ? 1 : 0;
+                for (int q = 0; q < rx.n; ++q)
+                    for (int w = ca[q] >> 5; 32 * w < cb[q]; ++w) {
+                        const int tq = T.rx.n == 2 && w >= T.w0[1] ? 1 : 0;
+                        const int at = staged ? T.row(tp, r) * T.words + T.word(tq, w) : 0;
+                        unsigned b = staged ? S.bits[at] : __ldcg(u.bits + (int64_t)r * P.words + w);
+                        if (32 * w < ca[q]) b &= 0xffffffffu << (ca[q] - 32 * w);
+                        if (cb[q] - 32 * w < 32) b &= (1u << (cb[q] - 32 * w)) - 1u;
+                        for (; b; b &= b - 1u) {
+                            const int bit = __ffs(b) - 1, xs = u.x0 + (32 * w + bit) * P.sx;
+                            apply(ys, xs, staged ? S.mm[32 * at + bit] : __ldcg(L.mm + (int64_t)ys * L.nx + xs));
+                        }
+                    }
+            }
+        }
+    }
+    if (!touched) return;
+    const float pref2 = (float)(2.0 * L.dip_pref);
+    const int64_t i0 = (int64_t)y * L.nx + x;
+    float mv[RX_V];
+    double ev[RX_V], pv[RX_V];
+#pragma unroll
+    for (int v = 0; v < RX_V; ++v) {
+        const bool t = (touched >> v) & 1u;
+        const int64_t i = i0 + (int64_t)v * nx;
+        mv[v] = t ? L.mm[i] : 0.f;
+        ev[v] = t ? L.E_dip[i] : 0.0;
+        pv[v] = t && Kp ? L.E_dip_perp[i] : 0.0;
+    }
+#pragma unroll
+    for (int v = 0; v < RX_V; ++v) {
+        if (mv[v] == 0.f) continue;                  // not touched, or nothing is added to an empty cell
+        const int64_t i = i0 + (int64_t)v * nx;
+        if ((neg >> v) & 1u) { ev[v] = -ev[v]; if (u.flip_perp) pv[v] = -pv[v]; }
+        L.E_dip[i] = ev[v] + (double)(pref2 * (mv[v] * acc[v]));
+        if (Kp) L.E_dip_perp[i] = pv[v] + (double)(pref2 * (mv[v] * accp[v]));
+    }
+}
+
+// Update of the tile of rows [ty0, ty1) and columns [tx0, tx1), by the whole CTA.
+HS_DEV void relax_update_tile(const HsLattice &L, const RelaxPlan &P, const SubUpdate &u, RelaxShared &S, int ty0, int ty1,
+                              int tx0, int tx1) {
+    RelaxTile T;
+    T.ry = reach_of(ty0, ty1 - 1, u.hy, u.wrap, L.ny);
+    T.rx = reach_of(tx0, tx1 - 1, u.hx, u.wrap, L.nx);
+    T.nr[1] = T.nw[1] = T.r0[1] = T.w0[1] = 0;
+    for (int p = 0; p < T.ry.n; ++p) { T.r0[p] = first_at(T.ry.a[p], u.y0, P.sy); T.nr[p] = past_at(T.ry.b[p], u.y0, P.sy) - T.r0[p]; }
+    for (int q = 0; q < T.rx.n; ++q) {
+        T.w0[q] = first_at(T.rx.a[q], u.x0, P.sx) >> 5;
+        T.nw[q] = ((past_at(T.rx.b[q], u.x0, P.sx) + 31) >> 5) - T.w0[q];
+    }
+    // wrapped ranges may share the word between them
+    if (T.rx.n == 2 && T.w0[1] < T.w0[0] + T.nw[0]) { T.nw[1] -= T.w0[0] + T.nw[0] - T.w0[1]; T.w0[1] = T.w0[0] + T.nw[0]; }
+    if (T.nw[1] < 0) T.nw[1] = 0;
+    T.rows = T.nr[0] + T.nr[1];
+    T.words = T.nw[0] + T.nw[1];
+    const int n = T.rows * T.words;
+    const bool staged = n <= RX_WORDS;
+    unsigned any = 0u;
+    for (int k = threadIdx.x; k < n; k += RX_T) {
+        const int tr = k / T.words, tw = k - tr * T.words;
+        const int r = tr < T.nr[0] ? T.r0[0] + tr : T.r0[1] + tr - T.nr[0];
+        const int w = tw < T.nw[0] ? T.w0[0] + tw : T.w0[1] + tw - T.nw[0];
+        const unsigned b = __ldcg(u.bits + (int64_t)r * P.words + w);
+        any |= b;
+        if (staged) S.bits[k] = b;
+    }
+    if (!__syncthreads_or(any != 0u)) return;      // no switch in reach
+    if (staged) {
+        auto place = [&](int k, int &r, int &w) {      // subgrid row and word of staged word k
+            const int tr = k / T.words, tw = k - tr * T.words;
+            r = tr < T.nr[0] ? T.r0[0] + tr : T.r0[1] + tr - T.nr[0];
+            w = tw < T.nw[0] ? T.w0[0] + tw : T.w0[1] + tw - T.nw[0];
+        };
+        auto moment = [&](int r, int w, int bit) {
+            return __ldcg(L.mm + (int64_t)(u.y0 + r * P.sy) * L.nx + u.x0 + (32 * w + bit) * P.sx);
+        };
+        if (threadIdx.x < 32) {       // the list, 32 words at a time, in order
+            int at = 0;
+            for (int k0 = 0; k0 < n; k0 += 32) {
+                const int k = k0 + (int)threadIdx.x;
+                unsigned b = k < n ? S.bits[k] : 0u;
+                int incl = __popc(b);
+                const int own = incl;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, incl, o); if ((int)threadIdx.x >= o) incl += t; }
+                int pos = at + incl - own, r = 0, w = 0;
+                if (b) place(k, r, w);
+                for (; b && pos < RX_LIST; b &= b - 1u, ++pos) {
+                    const int bit = __ffs(b) - 1;
+                    S.hit[pos] = RelaxHit{u.y0 + r * P.sy, u.x0 + (32 * w + bit) * P.sx, moment(r, w, bit)};
+                }
+                at += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (threadIdx.x == 0) S.n = at;
+        }
+        __syncthreads();
+        if (S.n > RX_LIST) {
+            for (int k = threadIdx.x; k < 32 * n; k += RX_T) {     // moments of the switches
+                if (!((S.bits[k >> 5] >> (k & 31)) & 1u)) continue;
+                int r, w;
+                place(k >> 5, r, w);
+                S.mm[k] = moment(r, w, k & 31);
+            }
+            __syncthreads();
+        }
+    }
+    const int gx = (tx1 - tx0 + 31) / 32, parts = gx * ((ty1 - ty0 + RX_V - 1) / RX_V);
+    for (int e = threadIdx.x >> 5; e < parts; e += RX_T / 32) {
+        const int y = ty0 + RX_V * (e / gx), x = tx0 + 32 * (e % gx);
+        if (u.kind == 2) relax_update_warp<true>(L, P, u, T, S, staged, y, x, ty1, tx1);
+        else relax_update_warp<false>(L, P, u, T, S, staged, y, x, ty1, tx1);
+    }
+    __syncthreads();       // the staging is free again; the next decisions read this CTA's energies
+}
+
+__global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCounters *C, RelaxBufs B, RelaxPlan P) {
+    extern __shared__ __align__(16) unsigned char s_rx_raw[];
+    RelaxShared &s_rx = *reinterpret_cast<RelaxShared *>(s_rx_raw);
+    __shared__ uint64_t s_key[RX_MAX_P];
+    __shared__ int s_order[RX_MAX_P];
+    __shared__ unsigned char s_active[RX_MAX_P];
+    __shared__ int s_w[RX_T / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n_sub = P.sx * P.sy;
+    for (int o = threadIdx.x; o < n_sub; o += RX_T) s_active[o] = L.occ[(int64_t)(o / P.sx) * L.nx + o % P.sx] != 0;
+    const int64_t N = (int64_t)L.nx * L.ny;
+    if (B.st->done) return;
+    int sweep = B.st->sweep, done = 0;
+    const uint64_t call0 = C->rng_call;
+    long long switched = 0;              // by this launch (every CTA counts)
+    unsigned nbar = 0, slot = 0;         // barriers passed, subgrids so far
+    unsigned seen[2] = {0u, 0u};
+    int made = 0;
+    bool ok = true;
+    for (; made < P.max_sweeps && !done && ok; ++made) {
+        // the subgrid order: a stable argsort of the sweep's variates
+        for (int e = threadIdx.x; e < n_sub; e += RX_T) s_key[e] = u53_bits(L.seed, call0 + made, (uint32_t)e);
+        __syncthreads();
+        for (int e = threadIdx.x; e < n_sub; e += RX_T) {
+            const uint64_t k = s_key[e];
+            int rank = 0;
+            for (int j = 0; j < n_sub; ++j) rank += (s_key[j] < k) || (s_key[j] == k && j < e);
+            s_order[rank] = e;
+        }
+        __syncthreads();
+        long long sweep_total = 0;
+        for (int i = 0; i < n_sub && ok; ++i) {
+            const int o = s_order[i];
+            const int y0 = o / P.sx, x0 = o % P.sx;
+            if (!s_active[o]) continue;
+            unsigned *bits = P.bits + (int64_t)(slot & 1) * P.rows * P.words;
+            // decisions: one word (32 candidates of a row) per warp
+            int mine = 0;
+            for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
+                const int ty0 = (t / P.tiles_x) * P.TY, w = t % P.tiles_x;
+                const int r0 = first_at(ty0, y0, P.sy), r1 = past_at(min(ty0 + P.TY, L.ny) - 1, y0, P.sy);
+                const int x = x0 + (32 * w + lane) * P.sx;
+                if (w >= P.words) continue;
+                for (int r = r0 + warp; r < r1; r += RX_T / 32) {
+                    const int y = y0 + r * P.sy;
+                    bool f = false;
+                    if (x < L.nx) {
+                        double E = 0.0, Ep;
+                        if (L.has_exchange) hs_energy_at(L, y, x, E, Ep);
+                        else {          // the operations of hs_energy_at on this CTA's own cells (through L1)
+                            const int64_t c = (int64_t)y * L.nx + x;
+                            if (L.has_dipolar) E += L.E_dip[c];
+                            if (L.zee) E += (double)L.m[c] * (double)__ldg(L.zee + c);
+                        }
+                        const double dE = -2.0 * E;
+                        f = P.ignore_barrier ? dE < 0.0 : dE / 2.0 + (double)L.E_B[(int64_t)y * L.nx + x] < 0.0;
+                    }
+                    const unsigned b = __ballot_sync(0xffffffffu, f);
+                    if (lane == 0) bits[(int64_t)r * P.words + w] = b;
+                    mine += __popc(b);
+                    if (f && !L.has_exchange) {
+                        const int64_t c = (int64_t)y * L.nx + x;
+                        L.m[c] = (int8_t)(-L.m[c]);
+                        L.mm[c] = -L.mm[c];
+                    }
+                }
+            }
+            mine = block_sum(lane == 0 ? mine : 0, s_w);
+            const int all = grid_barrier(P.g, nbar++, (unsigned)mine, seen, P.wait_ns);
+            ok = all >= 0;
+            if (L.has_exchange && ok) {
+                for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
+                    const int ty0 = (t / P.tiles_x) * P.TY, w = t % P.tiles_x;
+                    const int r0 = first_at(ty0, y0, P.sy), r1 = past_at(min(ty0 + P.TY, L.ny) - 1, y0, P.sy);
+                    if (w >= P.words) continue;
+                    for (int r = r0 + warp; r < r1; r += RX_T / 32)
+                        if ((bits[(int64_t)r * P.words + w] >> lane) & 1u) {
+                            const int64_t c = (int64_t)(y0 + r * P.sy) * L.nx + x0 + (32 * w + lane) * P.sx;
+                            L.m[c] = (int8_t)(-L.m[c]);
+                            L.mm[c] = -L.mm[c];
+                        }
+                }
+                ok = grid_barrier(P.g, nbar++, 0u, seen, P.wait_ns) >= 0;
+            }
+            if (!ok) break;
+            sweep_total += all;
+            if (all && L.has_dipolar) {
+                SubUpdate u;
+                u.y0 = y0; u.x0 = x0;
+                u.sub = hs_sub(L, y0, x0);
+                u.mode = all > L.trunc_cutoff ? 1 : 0;
+                u.flip_perp = !(L.dip_keep_perp_sign && all > 1);
+                u.bits = bits;
+                int wy, wx;
+                hs_window(L, u.mode, true, u.hy, wy);
+                hs_window(L, u.mode, false, u.hx, wx);
+                u.wrap = wy != 0;
+                u.kind = u.wrap ? (u.mode ? 2 : 1) : 0;
+                if (!u.wrap) { u.hy = min(u.hy, L.dip_wy); u.hx = min(u.hx, L.dip_wx); }   // the kernel ends there
+                for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
+                    const int ty0 = (t / P.tiles_x) * P.TY, tx0 = (t % P.tiles_x) * P.TX;
+                    const int ty1 = min(ty0 + P.TY, L.ny), tx1 = min(tx0 + P.TX, L.nx);
+                    relax_update_tile(L, P, u, s_rx, ty0, ty1, tx0, tx1);
+                }
+            }
+            ++slot;
+        }
+        if (!ok) break;
+        switched += sweep_total;
+        // the stop rule (relax_compare_kernel, relax_end_kernel)
+        if (sweep_total == 0) { done = 1; ++sweep; continue; }
+        int8_t *snap = B.snap + ((sweep + 1) & 1) * N;
+        int d = 0;
+        for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
+            const int ty0 = (t / P.tiles_x) * P.TY, tx0 = (t % P.tiles_x) * P.TX;
+            const int ty1 = min(ty0 + P.TY, L.ny), tw = min(tx0 + P.TX, L.nx) - tx0, n = (ty1 - ty0) * tw;
+            for (int e = threadIdx.x; e < n; e += RX_T) {
+                const int64_t c = (int64_t)(ty0 + e / tw) * L.nx + tx0 + e % tw;
+                const int8_t a = L.m[c];
+                d |= a != snap[c];
+                snap[c] = a;
+            }
+        }
+        d = block_sum(d, s_w);
+        const int differs = grid_barrier(P.g, nbar++, d ? 1u : 0u, seen, P.wait_ns);
+        ok = differs >= 0;
+        if (!ok) break;
+        ++sweep;
+        if (!differs || sweep >= P.n_max) done = 1;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        B.st->sweep = sweep;
+        B.st->done = done;
+        C->rng_call = call0 + made + (ok ? 0 : 1);
+        C->switches += switched;
+        C->attempted += switched;
+        C->n_sw = 0;
+        if (!ok) { C->status |= HS_ST_TIMEOUT; B.st->done = 1; }
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -647,6 +1082,48 @@ int hs_relax_check_impl(const HsLattice &L, HsCounters *C, int n_max, void *scra
     if ((rc = hs_check_launch("relax_compare_kernel"))) return rc;
     relax_end_kernel<<<1, 1, 0, st>>>(C, B, n_max);
     return hs_check_launch("relax_end_kernel");
+}
+
+int hs_relax_run_impl(const HsLattice &L, HsCounters *C, int ignore_barrier, int n_max, int max_sweeps, void *scratch,
+                      int64_t bytes, cudaStream_t st) {
+    int rc = check_common(L, "hs_relax_run", bytes);
+    if (rc) return rc;
+    RelaxBufs B;
+    layout(L, reinterpret_cast<char *>(scratch), &B);
+    RelaxPlan P{};
+    steps_of(L, 0, P.sx, P.sy);
+    if (P.sx > L.nx || P.sy > L.ny) { hs_set_error("hs_relax_run: lattice smaller than two unit cells"); return HS_EINVAL; }
+    int dev = 0, sms = 148, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaFuncSetAttribute(relax_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RelaxShared));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, relax_grid_kernel, RX_T, sizeof(RelaxShared));
+    if (e != cudaSuccess) { hs_set_error("hs_relax_run: %s", cudaGetErrorString(e)); return HS_ECUDA; }
+    P.TX = 32 * P.sx;
+    P.tiles_x = (L.nx + P.TX - 1) / P.TX;
+    // the shortest tiles that still give every SM at most one: a barrier costs less with fewer CTAs
+    P.TY = P.sy;
+    while ((int64_t)P.tiles_x * ((L.ny + P.TY - 1) / P.TY) > sms && P.TY < 64) P.TY += P.sy;
+    P.tiles = P.tiles_x * ((L.ny + P.TY - 1) / P.TY);
+    P.rows = (L.ny + P.sy - 1) / P.sy;
+    P.words = ((L.nx + P.sx - 1) / P.sx + 31) / 32;
+    P.ignore_barrier = ignore_barrier;
+    P.n_max = n_max;
+    P.max_sweeps = max_sweeps;
+    P.wait_ns = RX_WAIT_NS;
+    P.bits = reinterpret_cast<unsigned *>(B.cells);       // at most 4 N bytes: minimize()'s list
+    P.g = reinterpret_cast<RelaxGrid *>(B.hist);
+    static_assert(sizeof(RelaxGrid) <= 4 * MN_PASSES * MN_BINS, "the grid state lives in minimize()'s histograms");
+    if (8LL * P.rows * P.words > 4 * n_cells(L)) { hs_set_error("hs_relax_run: bitmap larger than its buffer"); return HS_ERANGE; }
+    e = cudaMemsetAsync(P.g, 0, sizeof(RelaxGrid), st);
+    if (e != cudaSuccess) { hs_set_error("hs_relax_run: %s", cudaGetErrorString(e)); return HS_ECUDA; }
+    HsLattice Lv = L;
+    void *args[] = {&Lv, &C, &B, &P};
+    const int grid = std::max(1, std::min(P.tiles, sms * std::max(per, 1)));
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(relax_grid_kernel), dim3(grid), dim3(RX_T), args,
+                                    sizeof(RelaxShared), st);
+    if (e != cudaSuccess) { hs_set_error("relax_grid_kernel: %s", cudaGetErrorString(e)); return HS_ECUDA; }
+    return hs_check_launch("relax_grid_kernel");
 }
 
 int hs_minimize_begin_impl(const HsLattice &L, void *scratch, int64_t bytes, cudaStream_t st) {

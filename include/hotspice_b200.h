@@ -51,6 +51,7 @@ extern "C" {
 #define HS_ST_SWITCH_OVERFLOW 2  /* more switches than the switch list holds               */
 #define HS_ST_POISSON_OVERFLOW 4 /* Poisson-disc grid/queue capacity exceeded              */
 #define HS_ST_WOLFF_OVERFLOW 8   /* Wolff frontier capacity exceeded                       */
+#define HS_ST_TIMEOUT        32  /* a grid barrier of hs_relax_run gave up                  */
 #define HS_ST_STEP_CAP       16  /* a device-armed progress() run used its whole per-launch step
                                     budget before its stop rule held (set by the next
                                     hs_progress_arm / hs_progress_disarm)                     */
@@ -282,6 +283,11 @@ int hs_relax_subset(const HsLattice *L, HsCounters *C, const HsSwitchList *sw, i
  * one two sweeps before, or n_max = int(sqrt(nx^2 + ny^2)) sweeps were made. */
 int hs_relax_check(const HsLattice *L, HsCounters *C, int32_t n_max, void *scratch, int64_t scratch_bytes,
                    void *stream);
+/* Up to max_sweeps sweeps (not simultaneous) with hs_relax_check's stop rule after each, in one
+ * cooperative launch; the same state as that many hs_minimize_all / hs_relax_check pairs, except that
+ * n_sw is 0 afterwards. Needs the whole launch resident at once (it waits for the GPU otherwise). */
+int hs_relax_run(const HsLattice *L, HsCounters *C, int32_t ignore_barrier, int32_t n_max, int32_t max_sweeps,
+                 void *scratch, int64_t scratch_bytes, void *stream);
 /* Start minimize(): clears the stop state and the per-magnet pick counts. */
 int hs_minimize_begin(const HsLattice *L, void *scratch, int64_t scratch_bytes, void *stream);
 /* One iteration of minimize(ignore_barrier=True) (core.py:771-797): with n magnets whose
