@@ -425,6 +425,7 @@ struct __align__(16) EngShared {
     union {
         struct { int q[ENG_NT / 32][NEEL_QCAP]; float lb[ENG_NT / 32][NEEL_QCAP]; } nq;   // owner path: candidates
         SwX sw[ENG_SWCAP];
+        WolffFast wolff;
     };
 };
 static_assert(sizeof(HsInstance) % 8 == 0, "HsInstance is copied in 8-byte words");
@@ -1058,7 +1059,7 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
             S.all();
         } else {  // Wolff
             if (rank == 0) {
-                wolff_step_cta(L, C, sw, wolff_scratch_of(L, I.scratch));
+                wolff_step_cta(L, C, sw, wolff_scratch_of(L, I.scratch), sh.wolff);
                 __syncthreads();
                 if (threadIdx.x == 0) decide_next(st + 1);
             }

@@ -18,7 +18,8 @@
 namespace {
 
 __global__ void __launch_bounds__(WT) wolff_kernel(HsLattice L, HsCounters *C, HsSwitchList sw, WolffScratch S) {
-    wolff_step_cta(L, C, sw, S);
+    __shared__ __align__(16) WolffFast s_fast;
+    wolff_step_cta(L, C, sw, S, s_fast);
 }
 
 }  // namespace

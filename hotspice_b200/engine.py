@@ -57,7 +57,7 @@ def step_model(mm: Magnets) -> tuple[float, float, float]:
     class (dense / half / sparse, which also carries the perpendicular channel of the in-plane
     lattices), Néel steps spread over the cluster like cs^0.85 (512 x 512 dense: 172 us on one CTA,
     16.5 us on 16; 64 x 64: 7.4 and 5.1 us) and Metropolis steps like cs^0.5; a Wolff step grows its
-    cluster on one CTA and costs 10-17 us above the critical temperature. Inside a full batch the
+    cluster on one CTA and costs about 6 us above the critical temperature. Inside a full batch the
     CTAs share the L2, so a batch's launch plan is best measured (:meth:`BatchEngine.tune_split`)."""
     n = mm.nx * mm.ny
     f = mm.n / max(n, 1)
@@ -67,7 +67,7 @@ def step_model(mm: Magnets) -> tuple[float, float, float]:
         c, beta = ((0.00184, 0.915), (0.0040, 0.807), (0.0111, 0.704))[cls]
         return 4.0, c * n ** beta, 0.85
     if sch == Scheme.WOLFF:
-        return 11.0 + 6e-6 * n, 0.0, 0.0
+        return 5.2 + 6e-6 * n, 0.0, 0.0
     c, beta = ((0.0037, 0.70), (0.0068, 0.70), (0.0061, 0.73))[cls]
     return 5.0, c * n ** beta, 0.5
 
