@@ -68,4 +68,34 @@ int hs_launch_engine(const HsInstance *insts, int n_inst, int cluster_size, int 
                      long long *elapsed_ns, cudaStream_t st);
 int hs_engine_max_clusters_impl(int cluster_size);
 
+#ifdef __CUDACC__
+// Launch with programmatic stream serialisation: the kernel may start while the one before it in the
+// stream still runs, if that one allows it (hs_pdl_begin's trigger), and must not touch global memory
+// before hs_pdl_begin, which waits until everything before it has finished and is visible. Used for
+// the kernels of a step, whose launch latencies are comparable to their run times.
+template <typename... P, typename... A>
+int hs_launch_step(const char *what, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    if (e != cudaSuccess) { hs_set_error("%s: %s", what, cudaGetErrorString(e)); return HS_ECUDA; }
+    return hs_check_launch(what);
+}
+
+// First statement of such a kernel, on every path: lets the next kernel start, then waits for the
+// ones before.
+__device__ __forceinline__ void hs_pdl_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+#endif
+
 inline int64_t hs_align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }

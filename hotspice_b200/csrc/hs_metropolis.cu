@@ -24,6 +24,7 @@ template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) metropolis_kernel(HsLattice L, HsCounters *C, HsSwitchList sw, HsGridPlan P,
                                                         MetroScratch S, int ws_bytes) {
     extern __shared__ __align__(16) unsigned char s_ws[];   // the Poisson-disc sampler's arrays, if given
+    hs_pdl_begin();
     metro_step_cta<THREADS == PT>(L, C, sw, P, S, ws_bytes > 0 ? s_ws : nullptr, ws_bytes);
 }
 
@@ -73,9 +74,14 @@ int hs_launch_metropolis(const HsLattice &L, HsCounters *C, const HsSwitchList &
             granted = (int)METRO_WS_MAX;
         }
     }
-    if (P.sample_scheme == HS_SAMPLE_POISSON) metropolis_kernel<PT><<<1, PT, ws, st>>>(L, C, sw, P, S, ws);
-    else metropolis_kernel<MT><<<1, MT, 0, st>>>(L, C, sw, P, S, 0);
-    int rc = hs_check_launch("metropolis_kernel");
+    int rc;
+    if (P.sample_scheme == HS_SAMPLE_POISSON) rc = hs_launch_step("metropolis_kernel", metropolis_kernel<PT>, 1, PT, ws, st, L, C, sw, P, S, ws);
+    else {
+        // a thread per candidate: every step code strides by the block, and a block of one or two
+        // warps starts and synchronises sooner than one of 32 (48 candidates: 7.0 -> 5.7 us)
+        const int threads = P.sample_scheme == HS_SAMPLE_GRID ? (int)std::min<int64_t>(MT, hs_align_up(P.n_sc, 32)) : 32;
+        rc = hs_launch_step("metropolis_kernel", metropolis_kernel<MT>, 1, threads, 0, st, L, C, sw, P, S, 0);
+    }
     if (rc) return rc;
     if (L.has_dipolar) return hs_launch_dipolar_update(L, sw, &C->n_sw, 0, HS_UPDATE_MULTIPLE, C, st);
     return HS_OK;

@@ -556,7 +556,18 @@ HS_DEV bool metro_grid_fast(const HsLattice &L, HsCounters *C, const HsSwitchLis
             x += ox; y += oy;
             ok = x >= 0 && x < L.nx && y >= 0 && y < L.ny;
         }
-        valid = ok && L.occ[(int64_t)y * L.nx + x] != 0;
+    }
+    // occupation, spin, moment and energies in one round trip
+    int8_t m_old = 0;
+    float mm_old = 0.f;
+    double E = 0.0, Ep;
+    if (ok) {
+        const int64_t i = (int64_t)y * L.nx + x;
+        const int8_t oc = __ldg(L.occ + i);
+        m_old = __ldcg(L.m + i);
+        mm_old = __ldcg(L.mm + i);
+        hs_energy_at(L, y, x, E, Ep);
+        valid = oc != 0;
     }
     int pre_ok, r, n_ok, k;
     block_excl_scan2(ok, valid, wt, pre_ok, r, n_ok, k);
@@ -568,15 +579,8 @@ HS_DEV bool metro_grid_fast(const HsLattice &L, HsCounters *C, const HsSwitchLis
     int acc = 0;
     double tpart = 0.0;
     long long near = 0;
-    int8_t m_old = 0;
-    float mm_old = 0.f;
     if (valid) {
         const int64_t i = (int64_t)y * L.nx + x;
-        // the spin and moment for the flip are loaded with the energies (one round trip)
-        m_old = __ldcg(L.m + i);
-        mm_old = __ldcg(L.mm + i);
-        double E, Ep;
-        hs_energy_at(L, y, x, E, Ep);
         const double beta = hs_beta(L, i);
         const double p = fmin(fmax(exp(2.0 * E * beta), 1e-10), 1e10);
         if (mtime) {
@@ -665,7 +669,18 @@ HS_DEV bool metro_grid_warp(const HsLattice &L, HsCounters *C, const HsSwitchLis
             x += ox; y += oy;
             ok = x >= 0 && x < L.nx && y >= 0 && y < L.ny;
         }
-        valid = ok && __ldg(L.occ + (int64_t)y * L.nx + x) != 0;
+    }
+    // occupation, spin, moment and energies in one round trip
+    int8_t m_old = 0;
+    float mm_old = 0.f;
+    double E = 0.0, Ep;
+    if (ok) {
+        const int64_t i = (int64_t)y * L.nx + x;
+        const int8_t oc = __ldg(L.occ + i);
+        m_old = __ldcg(L.m + i);
+        mm_old = __ldcg(L.mm + i);
+        hs_energy_at(L, y, x, E, Ep);
+        valid = oc != 0;
     }
     const unsigned below = (1u << lane) - 1u;
     const unsigned okb = __ballot_sync(0xffffffffu, ok), vb = __ballot_sync(0xffffffffu, valid);
@@ -678,15 +693,8 @@ HS_DEV bool metro_grid_warp(const HsLattice &L, HsCounters *C, const HsSwitchLis
     int acc = 0;
     double tpart = 0.0;
     int near = 0;
-    int8_t m_old = 0;
-    float mm_old = 0.f;
     if (valid) {
         const int64_t i = (int64_t)y * L.nx + x;
-        // the spin and moment for the flip are loaded with the energies (one round trip)
-        m_old = __ldcg(L.m + i);
-        mm_old = __ldcg(L.mm + i);
-        double E, Ep;
-        hs_energy_at(L, y, x, E, Ep);
         const double beta = hs_beta(L, i);
         const double p = fmin(fmax(exp(2.0 * E * beta), 1e-10), 1e10);
         if (mtime) {
