@@ -988,6 +988,27 @@ class Magnets(ABC):
             rc = self._lib.hs_wolff_step(L, C, s, buf.data_ptr(), buf.numel(), stream)
         _lib.check(rc, f'hs_{kind}_step')
 
+    def _step_switches(self):
+        """Number of switches of the step just launched and their (2, n) indices, read with one wait:
+        the counters and a list of up to 1024 entries go to pinned memory side by side (a longer
+        list's entries are read once their number is known)."""
+        t = self._sw[0]
+        cap = t.shape[1]
+        whole = cap <= 1024
+        nc = self._counters.numel()
+        host = getattr(self, '_step_host', None)
+        if host is None or host.numel() < nc + (8 * cap if whole else 0):
+            host = self._step_host = torch.empty(nc + (8 * cap if whole else 0), dtype=torch.uint8, pin_memory=True)
+        host[:nc].copy_(self._counters, non_blocking=True)
+        if whole:
+            host[nc:nc + 8 * cap].view(torch.int32).copy_(t[:2].view(-1), non_blocking=True)
+        torch.cuda.current_stream(self.device).synchronize()
+        raw = host.numpy()
+        n = int(raw[:nc].view(_lib.COUNTERS_DTYPE)[0]['n_sw'])
+        if whole:
+            return n, raw[nc:nc + 8 * cap].view(np.int32).reshape(2, cap)[:, :n].astype(np.int64)
+        return n, t[:2, :n].cpu().numpy().astype(np.int64)
+
     def update(self, *args, **kwargs):
         """One update step (hotspice/core.py:604-622). Returns the switched index/indices."""
         if self._T_zero:
@@ -997,18 +1018,12 @@ class Magnets(ABC):
                 warnings.warn("T=0 somewhere in the domain, so ergodicity can not be guaranteed. Proceed with caution.", stacklevel=2)
             return None
         if self.params.UPDATE_SCHEME == Scheme.NEEL:
-            self._write_counters(t_max=float(kwargs.get('t_max', 1)), progress=0, done=0)
+            self._set_control(t_max=float(kwargs.get('t_max', 1)), progress=0, done=0)
         args_ = self._step_args(kwargs)
         self._launch(args_, self._stream())
-        c = self._read_counters()
-        n = int(c['n_sw'])
-        t, _ = self._sw
+        n, idx = self._step_switches()
         if self.params.UPDATE_SCHEME == Scheme.NEEL:
-            if n == 0:
-                return None
-            yx = t[:2, 0].cpu().numpy()
-            return (int(yx[0]), int(yx[1]))
-        idx = t[:2, :n].cpu().numpy().astype(np.int64)
+            return (int(idx[0, 0]), int(idx[1, 0])) if n else None
         if self.params.UPDATE_SCHEME == Scheme.WOLFF:
             order = np.lexsort((idx[1], idx[0]))
             idx = idx[:, order]
