@@ -516,30 +516,9 @@ dip_update_persist_kernel(HsLattice L, HsSwitchList sw, const int32_t *n_sw_dev,
     }
 }
 
-// Update of a short list (up to FEW_MAX switches): work follows the switches instead of the lattice.
-// An item is 32 columns x 8 rows of one switch's window, one warp's work (a lane has a column, so a
-// kernel row is read by consecutive lanes); the items of all switches are numbered through and
-// dealt to the warps. A cell in several windows belongs to the first of them in list order; its
-// item adds the later ones' contributions in order, so the sums are those of dip_update_kernel bit
-// for bit. The common item meets no other window and reads nothing but its own cells and kernel rows.
-// Measured on B200 (cutoff 20a, 79 x 79 windows): us per step of two kernels, 512 x 512
-// 7.7 -> 6.7 and 1500 x 1201 with about 20 switches 18.6 -> 10.8; bound by the latencies of list,
-// moments, cells and the two launches.
-constexpr int FEW_MAX = 64, FEW_ITEMS = 128, FEW_R = 8, FEW_T = 256;
+constexpr int FEW_R = 8, FEW_T = 256;
 
-struct FewSw {
-    int y, x, mode, sub;
-    float mm;
-    int hy, hx, kind;        // kind 0: plain window, 1: minimum image, 2: truncated and periodic (hs_contrib)
-    int ylo, nr, xlo, nc;    // window rows and columns (ylo, xlo may be negative where they wrap)
-    int end;                 // items of the switches up to this one
-};
-
-HS_DEV bool few_covers(const HsLattice &L, const FewSw &w, int y, int x) {
-    if (w.kind == 0) return abs(y - w.y) <= w.hy && abs(x - w.x) <= w.hx;
-    return hs_axis_overlap(w.y, w.hy, 1, L.ny, y, 1) && hs_axis_overlap(w.x, w.hx, 1, L.nx, x, 1);
-}
-
+// few_stage / few_items over the whole GPU.
 __global__ void __launch_bounds__(FEW_T, 1)
 dip_update_few_kernel(HsLattice L, HsSwitchList sw, const int32_t *n_sw_dev, int n_host, int semantics,
                       const HsCounters *C, int cap) {
@@ -548,146 +527,14 @@ dip_update_few_kernel(HsLattice L, HsSwitchList sw, const int32_t *n_sw_dev, int
     __shared__ int s_w[FEW_T / 32];
     hs_pdl_begin();
     if (C && C->done) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nx = L.nx, ny = L.ny;
-    // stage the list (FEW_MAX <= FEW_T entries, loaded beside their number) with the switches' items
-    FewSw w{};
+    FewSw w{};       // loaded beside the number of switches (FEW_MAX <= FEW_T)
     if ((int)threadIdx.x < cap) {
         w.y = sw.y[threadIdx.x]; w.x = sw.x[threadIdx.x]; w.mode = sw.mode ? sw.mode[threadIdx.x] : 0;
     }
     const int nsw = min(n_sw_dev ? *n_sw_dev : n_host, cap);
     if (nsw <= 0) return;
-    const int k = threadIdx.x;
-    int items = 0;
-    if (k < nsw) {
-        w.sub = hs_sub(L, w.y, w.x);
-        w.mm = L.mm[(int64_t)w.y * nx + w.x];
-        int wy, wx;
-        hs_window(L, w.mode, true, w.hy, wy);
-        hs_window(L, w.mode, false, w.hx, wx);
-        w.kind = wy ? (w.mode ? 2 : 1) : 0;
-        if (w.sub < 0) { w.hy = w.hx = 0; w.kind = 0; }      // no kernel: only the sign flip of E applies
-        if (w.kind == 0) {
-            // a truncated plain window ends where the kernel does
-            if (w.sub >= 0) { w.hy = min(w.hy, L.dip_wy); w.hx = min(w.hx, L.dip_wx); }
-            w.ylo = max(0, w.y - w.hy); w.nr = min(ny - 1, w.y + w.hy) - w.ylo + 1;
-            w.xlo = max(0, w.x - w.hx); w.nc = min(nx - 1, w.x + w.hx) - w.xlo + 1;
-        } else {
-            if (2 * w.hy + 1 >= ny) { w.ylo = 0; w.nr = ny; } else { w.ylo = w.y - w.hy; w.nr = 2 * w.hy + 1; }
-            if (2 * w.hx + 1 >= nx) { w.xlo = 0; w.nc = nx; } else { w.xlo = w.x - w.hx; w.nc = 2 * w.hx + 1; }
-        }
-        if (w.sub >= 0 || semantics == HS_UPDATE_MULTIPLE)
-            items = ((w.nr + FEW_R - 1) / FEW_R) * ((w.nc + 31) / 32);
-    }
-    int incl = items;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
-    if (lane == 31) s_w[warp] = incl;
-    __syncthreads();
-    int before = 0, n_items = 0;
-#pragma unroll
-    for (int q = 0; q < FEW_T / 32; ++q) { if (q < warp) before += s_w[q]; n_items += s_w[q]; }
-    if (k < nsw) { w.end = before + incl; s_sw[k] = w; }
-    __syncthreads();
-    const bool two = L.use_perp != 0, flip_perp = !(L.dip_keep_perp_sign && nsw > 1);
-    const float pref2 = (float)(2.0 * L.dip_pref);
-    const int KW = 2 * L.dip_wx + 1, KH = 2 * L.dip_wy + 1;
-    const float *const Kg = L.K, *const Kpg = L.Kpo, *const mmg = L.mm;
-    double *const Eg = L.E_dip, *const Epg = L.E_dip_perp;
-    for (int item = blockIdx.x * (FEW_T / 32) + warp; item < n_items; item += gridDim.x * (FEW_T / 32)) {
-        int k = 0;                         // the switch: how many end at or before the item
-        for (int b = 0; b < nsw; b += 32)
-            k += __popc(__ballot_sync(0xffffffffu, b + lane < nsw && s_sw[b + lane].end <= item));
-        const FewSw own = s_sw[k];
-        const int tc_n = (own.nc + 31) / 32, tile = item - (k ? s_sw[k - 1].end : 0);
-        const int tr = tile / tc_n, tc = tile - tr * tc_n;
-        const int y0 = own.ylo + FEW_R * tr, x0 = own.xlo + 32 * tc, nr = min(FEW_R, own.nr - FEW_R * tr);
-        const int ncol = min(32, own.nc - 32 * tc);
-        int x = x0 + lane;
-        const bool inx = lane < ncol;
-        x = x < 0 ? x + nx : (x >= nx ? x - nx : x);
-        // the cells' energies and moments first: their loads complete while the sums are formed
-        float mv[FEW_R];
-        double ev[FEW_R], pv[FEW_R];
-        int row[FEW_R];
-#pragma unroll
-        for (int v = 0; v < FEW_R; ++v) {
-            int y = y0 + v;
-            y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
-            row[v] = y;
-            const bool in = inx && v < nr;
-            const int64_t i = (int64_t)y * nx + x;
-            mv[v] = in ? mmg[i] : 0.f;
-            ev[v] = in ? Eg[i] : 0.0;
-            pv[v] = in && two ? Epg[i] : 0.0;
-        }
-        float acc[FEW_R] = {}, accp[FEW_R] = {};
-        unsigned mine = inx ? (1u << nr) - 1u : 0u, neg = 0u;
-        auto apply = [&](const FewSw &w, bool all_in) {
-            const int dx0 = x - w.x;
-            if (w.kind == 0 && all_in) {   // the item's own plain window: every cell lies in it
-                const float *K = Kg + ((int64_t)max(w.sub, 0) * KH + (row[0] - w.y + L.dip_wy)) * KW + (dx0 + L.dip_wx);
-                const float *Kp = two ? Kpg + (K - Kg) : nullptr;
-                float kv[FEW_R], kp[FEW_R];
-#pragma unroll
-                for (int v = 0; v < FEW_R; ++v) {
-                    const bool in = inx && v < nr && w.sub >= 0;
-                    kv[v] = in ? __ldg(K + v * KW) : 0.f;
-                    kp[v] = in && two ? __ldg(Kp + v * KW) : 0.f;
-                    if (dx0 == 0 && row[v] == w.y) neg |= 1u << v;
-                }
-#pragma unroll
-                for (int v = 0; v < FEW_R; ++v) { acc[v] += w.mm * kv[v]; accp[v] += w.mm * kp[v]; }
-                return;
-            }
-#pragma unroll
-            for (int v = 0; v < FEW_R; ++v) {
-                if (!inx || v >= nr || !(all_in || few_covers(L, w, row[v], x))) continue;
-                if (dx0 == 0 && row[v] == w.y) neg |= 1u << v;
-                if (w.sub < 0) continue;
-                if (w.kind == 2) { hs_contrib(L, SwInfo{w.y, w.x, w.mode, w.sub, w.mm}, row[v], x, acc[v], accp[v]); continue; }
-                acc[v] += w.mm * hs_kval(L, Kg, w.sub, row[v] - w.y, dx0);
-                if (two) accp[v] += w.mm * hs_kval(L, Kpg, w.sub, row[v] - w.y, dx0);
-            }
-        };
-        // windows that may meet the item, in list order
-        const bool wraps = y0 < 0 || y0 + nr > ny || x0 < 0 || x0 + ncol > nx;
-        for (int b = 0; b < nsw; b += 32) {
-            bool meets = false;
-            if (b + lane < nsw) {
-                const FewSw &w = s_sw[b + lane];
-                meets = b + lane == k || wraps ||
-                        (hs_axis_overlap(w.y, w.hy, w.kind != 0, ny, y0, nr) && hs_axis_overlap(w.x, w.hx, w.kind != 0, nx, x0, ncol));
-            }
-            for (unsigned m = __ballot_sync(0xffffffffu, meets); m; m &= m - 1u) {
-                const int q = b + __ffs(m) - 1;
-                if (q == k) { apply(own, true); continue; }
-                const FewSw w = s_sw[q];
-                if (w.sub < 0 && semantics != HS_UPDATE_MULTIPLE) continue;
-                if (q > k) { apply(w, false); continue; }
-#pragma unroll
-                for (int v = 0; v < FEW_R; ++v)
-                    if (((mine >> v) & 1u) && few_covers(L, w, row[v], x)) mine &= ~(1u << v);   // an earlier window's cell
-            }
-        }
-#pragma unroll
-        for (int v = 0; v < FEW_R; ++v) {
-            if (!((mine >> v) & 1u)) continue;
-            const bool ng = (neg >> v) & 1u;
-            const double de = (double)(pref2 * (mv[v] * acc[v])), dp = (double)(pref2 * (mv[v] * accp[v]));
-            double e = ev[v], p = pv[v];
-            if (semantics == HS_UPDATE_MULTIPLE) {
-                if (ng) { e = -e; if (flip_perp) p = -p; }
-                e += de; p += dp;
-            } else {
-                e += de; p += dp;
-                if (ng) { e = -e; p = -p; }
-            }
-            const int64_t i = (int64_t)row[v] * nx + x;
-            Eg[i] = e;
-            if (two) Epg[i] = p;
-        }
-    }
+    const int n_items = few_stage<FEW_R>(L, w, nsw, semantics, s_sw, s_w);
+    few_items<FEW_R>(L, s_sw, nsw, n_items, semantics, blockIdx.x * (FEW_T / 32) + (threadIdx.x >> 5), gridDim.x * (FEW_T / 32));
 }
 
 // Direct-sum full recompute, one thread per target cell (hotspice/energies.py:290-308):

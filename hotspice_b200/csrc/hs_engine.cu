@@ -15,7 +15,8 @@
 // Every branch that decides how many barriers are executed is taken on values every CTA of
 // the cluster reads after a barrier, so all CTAs always execute the same barrier sequence.
 //
-// The dipolar update distributes work items (switch k, window row, 128-column segment) over
+// The dipolar update of up to FEW_MAX switches distributes pieces of their windows (few_items); a
+// longer list's distributes work items (switch k, window row, 128-column segment) over
 // all warps of the cluster. A strip (row, segment) is processed by the item of the first
 // switch whose window covers it, which accumulates the contributions of every covering
 // switch in list order: each strip is written once, deterministically, and the work is
@@ -40,6 +41,7 @@ namespace {
 #endif
 constexpr int ENG_NT = HS_ENGINE_THREADS;   // threads per CTA
 constexpr int ENG_MIN_CTAS = 65536 / (ENG_NT * HS_ENGINE_REGS);  // resident CTAs per SM at that register budget
+constexpr int ENG_FEW_R = 4;    // rows per item of a short list: 128 registers hold four rows' cells
 constexpr int ENG_SWCAP = 512;  // switches staged per CTA in shared memory
 constexpr int ENG_WS_MAX = HS_ENGINE_WS_MAX;  // largest dynamic shared workspace a launch may ask for
 
@@ -420,11 +422,13 @@ struct __align__(16) EngShared {
     int go[2];                          // step st runs while go[st & 1] (double-buffered)
     float mm1;
     double thr[2];                      // owner path: a key below thr[st & 1] switches for certain
+    int few_w[FEW_MAX / 32];
     float tw[32];                       // owner path: the warps' bounds
     int rowpre[NEEL_OWN_UY + 1];        // owner path: occupied cells before row y of a period of uy rows
     union {
         struct { int q[ENG_NT / 32][NEEL_QCAP]; float lb[ENG_NT / 32][NEEL_QCAP]; } nq;   // owner path: candidates
         SwX sw[ENG_SWCAP];
+        FewSw few[FEW_MAX];
         WolffFast wolff;
     };
 };
@@ -997,8 +1001,19 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
             S.all();
             if (L.has_dipolar) {
                 const int nsw = sh.nsw;
-                const int n = stage_switches(L, sw, nsw, sh.sw);
-                update_items(L, sh.sw, n, HS_UPDATE_MULTIPLE, rank * nwarps + warp, SCS * nwarps, sw, nsw);
+                if (nsw > 0 && nsw <= FEW_MAX) {       // uniform over the instance's threads
+                    FewSw w{};
+                    if ((int)threadIdx.x < nsw) {
+                        w.y = __ldcg(sw.y + threadIdx.x);
+                        w.x = __ldcg(sw.x + threadIdx.x);
+                        w.mode = sw.mode ? __ldcg(sw.mode + threadIdx.x) : 0;
+                    }
+                    const int items = few_stage<ENG_FEW_R>(L, w, nsw, HS_UPDATE_MULTIPLE, sh.few, sh.few_w);
+                    few_items<ENG_FEW_R>(L, sh.few, nsw, items, HS_UPDATE_MULTIPLE, rank * nwarps + warp, SCS * nwarps);
+                } else if (nsw > 0) {
+                    const int n = stage_switches(L, sw, nsw, sh.sw);
+                    update_items(L, sh.sw, n, HS_UPDATE_MULTIPLE, rank * nwarps + warp, SCS * nwarps, sw, nsw);
+                }
             }
             S.all();
         } else if (scheme == HS_SCHEME_NEEL) {

@@ -68,8 +68,8 @@ def step_model(mm: Magnets) -> tuple[float, float, float]:
         return 4.0, c * n ** beta, 0.85
     if sch == Scheme.WOLFF:
         return 5.2 + 6e-6 * n, 0.0, 0.0
-    c, beta = ((0.0037, 0.70), (0.0068, 0.70), (0.0061, 0.73))[cls]
-    return 5.0, c * n ** beta, 0.5
+    c, beta = ((0.00132, 0.65), (0.0010, 0.75), (0.0009, 0.82))[cls]
+    return 4.0, c * n ** beta, 0.5
 
 
 def model_time(m, cs):
