@@ -372,6 +372,12 @@ int hs_engine_run_ws(const HsInstance *insts, int32_t n_inst, int32_t cluster_si
                             reinterpret_cast<long long *>(elapsed_ns), (cudaStream_t)stream);
 }
 
+int hs_engine_controls(const HsInstance *insts, int32_t n_inst, double t_max, void *stream) {
+    if (!insts || n_inst < 0) { hs_set_error("hs_engine_controls: bad arguments"); return HS_EINVAL; }
+    if (n_inst == 0) return HS_OK;
+    return hs_engine_controls_impl(insts, n_inst, t_max, (cudaStream_t)stream);
+}
+
 int hs_engine_max_clusters(int32_t cluster_size) { return hs_engine_max_clusters_impl(cluster_size); }
 
 int hs_exchange_energy(const HsLattice *L, float *E, float *E_perp, void *stream) {

@@ -1139,6 +1139,17 @@ __global__ void __launch_bounds__(ENG_NT, ENG_MIN_CTAS) engine_kernel(const HsIn
     }
 }
 
+// Run controls of every instance of a launch: one kernel in place of a small copy per field and
+// instance (256 instances: 4.6 ms of host time per run_from_host()).
+__global__ void engine_controls_kernel(const HsInstance *insts, int n, double t_max) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    HsCounters *C = insts[i].C;
+    C->progress = 0;
+    C->done = 0;
+    C->t_max = t_max;
+}
+
 template <int CS>
 cudaError_t engine_allow_ws(int bytes) {
     // opt in to the dynamic workspace: static (about 30 KB) plus dynamic shared memory above
@@ -1196,6 +1207,11 @@ int hs_launch_engine(const HsInstance *insts, int n_inst, int cluster_size, int 
         case 16: return launch_engine<16>(insts, n_inst, work, n_clusters, ws_bytes, elapsed_ns, st);
         default: hs_set_error("engine: cluster size must be 1, 2, 4, 8 or 16"); return HS_EINVAL;
     }
+}
+
+int hs_engine_controls_impl(const HsInstance *insts, int n_inst, double t_max, cudaStream_t st) {
+    engine_controls_kernel<<<(n_inst + 127) / 128, 128, 0, st>>>(insts, n_inst, t_max);
+    return hs_check_launch("engine_controls_kernel");
 }
 
 int hs_engine_max_clusters_impl(int cluster_size) {

@@ -66,6 +66,7 @@ int hs_segments_copy_impl(void *staged, const HsSegment *segs, int n, int to_dev
 
 int hs_launch_engine(const HsInstance *insts, int n_inst, int cluster_size, int n_clusters, int *work, int ws_bytes,
                      long long *elapsed_ns, cudaStream_t st);
+int hs_engine_controls_impl(const HsInstance *insts, int n_inst, double t_max, cudaStream_t st);
 int hs_engine_max_clusters_impl(int cluster_size);
 
 #ifdef __CUDACC__

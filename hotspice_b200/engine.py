@@ -492,9 +492,9 @@ class BatchEngine:
                     if k == int(resync_every):
                         mm.resync_energies()
             return prepared
-        kws = [dict(kwargs) for _ in self.magnets]
-        for mm, kw in zip(self.magnets, kws):
-            mm._set_control(progress=0, done=0, t_max=float(kw.pop('t_max', math.inf)))
+        kws = [{k: v for k, v in kwargs.items() if k != 't_max'} for _ in self.magnets]
+        controls = {'progress': 0, 'done': 0, 't_max': float(kwargs.get('t_max', math.inf))}
+        stale = [mm for mm in self.magnets if getattr(mm, '_ctl', None) != controls]
         key = (tuple(steps), tuple(sorted((k, float(v)) for k, v in kwargs.items() if k != 't_max')),
                tuple(mm._version for mm in self.magnets), tuple(id(mm) for mm in self.magnets),
                tuple(sizes) if sizes else None, tuple(one_cta) if one_cta else None, self.cluster_size,
@@ -502,6 +502,15 @@ class BatchEngine:
         if self._cache is None or self._cache[0] != key:
             self._cache = (key, self._prepare(steps, kws, sizes, costs, one_cta))
         prepared = self._cache[1]
+        if len(stale) <= 2:
+            for mm in stale:
+                mm._set_control(**controls)
+        else:           # one launch per group sets every instance's
+            st = torch.cuda.current_stream(self.device).cuda_stream
+            for p in prepared:
+                _lib.check(self.lib.hs_engine_controls(p.inst.data_ptr(), p.n, controls['t_max'], st), 'hs_engine_controls')
+            for mm in self.magnets:
+                mm._ctl = dict(controls)
         self.launch(prepared)
         return prepared
 
@@ -644,8 +653,8 @@ class BatchEngine:
         ONE device to host copy). Asynchronous: synchronise the stream before reading host_out.
         With ``slot=`` the state was already sent by :meth:`upload` (the copy overlapped earlier
         work) and ``host_in`` may be omitted.
-        The run controls (progress, done, t_max) come from the loaded counters; :meth:`run` writes
-        only the ones that differ from what it needs."""
+        The run controls (progress, done, t_max) come from the loaded counters; :meth:`run` sets
+        them where they differ from what it needs."""
         st = torch.cuda.current_stream(self.device)
         segs, n, total, lay = self._segments(in_fields)
         if slot is None:

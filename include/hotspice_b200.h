@@ -363,6 +363,9 @@ int hs_engine_run(const HsInstance *insts, int32_t n_inst, int32_t cluster_size,
  * wall time (ns) its cluster spent on it in this launch, from claim to counter write-back. */
 int hs_engine_run_ws(const HsInstance *insts, int32_t n_inst, int32_t cluster_size, int32_t n_clusters,
                      int32_t *work, int32_t ws_bytes, int64_t *elapsed_ns, void *stream);
+/* Run controls of every instance of a launch (device descriptors, as hs_engine_run_ws takes them):
+ * progress = 0, done = 0, t_max. */
+int hs_engine_controls(const HsInstance *insts, int32_t n_inst, double t_max, void *stream);
 /* Number of clusters of `cluster_size` CTAs that can be resident at once (occupancy query). */
 int hs_engine_max_clusters(int32_t cluster_size);
 
