@@ -145,12 +145,21 @@ def split_makespan(cluster_runs, cta_runs, n_clusters, cs):
     return max(ctas)
 
 
+# Device time of a run on one CTA of a split launch over the model's. Measured on a batch of 256
+# mixed lattices: Néel runs 1.08 beside clusters of 2 and 1.13 beside clusters of 4 (Metropolis 1.13
+# and 1.36), cluster runs 0.95 to 1.02; every run on one CTA: 1.0. With it the plans of seven batches
+# (256 mixed, halves and a quarter of them, one scheme, one lattice class) ran 0.90, 0.89, 1.03, 0.96,
+# 0.96, 0.95 and 0.91 times as long as without; 1.12 and 1.3 gave 1.12 times on one of them.
+SPLIT_LOAD = {2: 1.1, 4: 1.2}
+
+
 def plan_split(models, steps, workers, sizes=CLUSTER_SIZES):
     """Cluster size and per-instance mode of one launch: the k longest runs (by their time on
     one CTA) use whole clusters of ``cs`` CTAs, the others one CTA each (the engine's split
     mode). Every size and a grid of k (k = n: one size for all) are simulated with
     :func:`split_makespan` over the modelled run times; ``workers[cs]`` is the number of
-    resident clusters of each size. Returns (cs, one_cta flags, modelled makespan in us)."""
+    resident clusters of each size. A run on one CTA beside cluster runs takes longer than in a
+    launch without clusters (SPLIT_LOAD). Returns (cs, one_cta flags, modelled makespan in us)."""
     t = model_time
     n = len(models)
     d1 = [st * t(m, 1) for m, st in zip(models, steps)]
@@ -161,8 +170,9 @@ def plan_split(models, steps, workers, sizes=CLUSTER_SIZES):
         if cs == 1:
             continue
         dc = [st * t(m, cs) for m, st in zip(models, steps)]
+        load = SPLIT_LOAD.get(cs, SPLIT_LOAD[4])
         for k in ks:
-            mk = split_makespan([dc[i] for i in order[:k]], [d1[i] for i in order[k:]], workers[cs], cs)
+            mk = split_makespan([dc[i] for i in order[:k]], [load * d1[i] for i in order[k:]], workers[cs], cs)
             if mk < best[0] * 0.99:
                 best = (mk, cs, k)
     mk, cs, k = best
