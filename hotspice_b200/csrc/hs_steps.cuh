@@ -1284,7 +1284,7 @@ HS_DEV void wolff_grow_warp(const HsLattice &L, WolffFast &F, int seed, uint64_t
 // the whole CTA and the stamps in the scratch. Engine, 300 x 300 periodic: 15.2 -> 5.8 us per step,
 // bound by the latencies of the chain (two Philox calls, two spin loads, the hash, per layer).
 HS_DEV void wolff_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList &sw, const WolffScratch &S, WolffFast &F) {
-    __shared__ int s_ncand, s_nacc, s_epoch;
+    __shared__ int s_ncand, s_nacc[2], s_epoch;   // s_nacc: by layer parity, so a late reader never meets the next layer's reset
     if (C->done) return;
     if (!hs_progress_continue(C, L.n_occ)) {
         if (threadIdx.x == 0) { C->done = 1; C->n_sw = 0; }
@@ -1336,7 +1336,7 @@ HS_DEV void wolff_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
     const int ch = L.nn_h / 2, cw = L.nn_w / 2;
     __syncthreads();
     for (; layer <= (int)N + 1; ++layer) {
-        if (threadIdx.x == 0) { s_ncand = 0; s_nacc = 0; }
+        if (threadIdx.x == 0) { s_ncand = 0; s_nacc[layer & 1] = 0; }
         __syncthreads();
         // frontier: unchecked same-spin cells j with q = j + c - b for a new cell q, mask[b] != 0
         for (int t = lstart + threadIdx.x; t < lend; t += blockDim.x) {
@@ -1376,13 +1376,13 @@ HS_DEV void wolff_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
             if (!(u > bond)) {
                 S.cl_ep[j] = epoch;
                 S.cl_layer[j] = layer;
-                S.list[lend + atomicAdd(&s_nacc, 1)] = j;
+                S.list[lend + atomicAdd(&s_nacc[layer & 1], 1)] = j;
             }
         }
         call += 1;
         __syncthreads();
         lstart = lend;
-        lend += s_nacc;
+        lend += s_nacc[layer & 1];
     }
     if (layer > (int)N + 1 && threadIdx.x == 0) C->status |= HS_ST_WOLFF_OVERFLOW;
     // flip the cluster; counters as in core.py:714-716
