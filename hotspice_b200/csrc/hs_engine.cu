@@ -401,7 +401,6 @@ HS_DEV WolffScratch wolff_scratch_of(const HsLattice &L, void *base) {
     WolffScratch S;
     S.chk_ep = reinterpret_cast<int32_t *>(p); p += hs_align_up_d(4 * N, 256);
     S.cl_ep = reinterpret_cast<int32_t *>(p); p += hs_align_up_d(4 * N, 256);
-    S.cl_layer = reinterpret_cast<int32_t *>(p); p += hs_align_up_d(4 * N, 256);
     S.list = reinterpret_cast<int32_t *>(p); p += hs_align_up_d(4 * N, 256);
     S.cand = reinterpret_cast<int32_t *>(p); p += hs_align_up_d(4 * N, 256);
     S.epoch = reinterpret_cast<int32_t *>(p);

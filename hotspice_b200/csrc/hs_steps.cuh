@@ -1136,8 +1136,7 @@ constexpr int WT = 1024;
 
 struct WolffScratch {
     int32_t *chk_ep;   // epoch in which the cell was checked (seed or frontier)
-    int32_t *cl_ep;    // epoch in which the cell joined the cluster
-    int32_t *cl_layer; // layer in which it joined
+    int32_t *cl_ep;    // epoch in which the cell joined the cluster, written when its layer is complete
     int32_t *list;     // cluster cells in BFS order (capacity N)
     int32_t *cand;     // frontier of the current layer (capacity N)
     int32_t *epoch;    // last epoch used with these stamps; kept here, not in the counters, so that
@@ -1327,9 +1326,8 @@ HS_DEV void wolff_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
         const int j = F.key[h];
         if (j < 0) continue;
         S.chk_ep[j] = epoch;
-        if (F.layer[h] >= 0) { S.cl_ep[j] = epoch; S.cl_layer[j] = F.layer[h]; }
     }
-    for (int t = threadIdx.x; t < F.lend; t += blockDim.x) S.list[t] = F.cell[t];
+    for (int t = threadIdx.x; t < F.lend; t += blockDim.x) { S.list[t] = F.cell[t]; S.cl_ep[F.cell[t]] = epoch; }
     const int8_t ms = L.m[F.cell[0]];
     uint64_t call = F.call;
     int lstart = F.lstart, lend = F.lend, layer = F.layers;
@@ -1338,9 +1336,11 @@ HS_DEV void wolff_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
     for (; layer <= (int)N + 1; ++layer) {
         if (threadIdx.x == 0) { s_ncand = 0; s_nacc[layer & 1] = 0; }
         __syncthreads();
-        // frontier: unchecked same-spin cells j with q = j + c - b for a new cell q, mask[b] != 0
+        // frontier: unchecked same-spin cells j with q = j + c - b for a new cell q, mask[b] != 0; the
+        // new cells are stamped here, so that no stamp changes while the bonds below read them
         for (int t = lstart + threadIdx.x; t < lend; t += blockDim.x) {
             const int q = S.list[t];
+            S.cl_ep[q] = epoch;
             const int qy = q / nx, qx = q % nx;
             for (int a = 0; a < L.nn_h; ++a)
                 for (int b = 0; b < L.nn_w; ++b) {
@@ -1369,13 +1369,11 @@ HS_DEV void wolff_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
                     if (L.pbc) { yy = hs_wrap(yy, ny); xx = hs_wrap(xx, nx); }
                     else if (yy < 0 || yy >= ny || xx < 0 || xx >= nx) continue;
                     const int k = yy * nx + xx;
-                    if (S.cl_ep[k] == epoch && S.cl_layer[k] < layer) count += w;
+                    if (S.cl_ep[k] == epoch) count += w;
                 }
             const double bond = wolff_bond_of(L, j, count);
             const double u = hs_u53(L.seed, call, (uint32_t)j);
             if (!(u > bond)) {
-                S.cl_ep[j] = epoch;
-                S.cl_layer[j] = layer;
                 S.list[lend + atomicAdd(&s_nacc[layer & 1], 1)] = j;
             }
         }

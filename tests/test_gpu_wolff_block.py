@@ -1,5 +1,6 @@
 """Wolff clusters that the whole CTA grows, over tens of layers, against the oracle: every layer's
-count of joined cells is read by all warps and set to zero again for a later layer."""
+count of joined cells is read by all warps and set to zero again for a later layer, and a cell that
+joins a layer must not count as a neighbour of that layer's other candidates."""
 import numpy as np
 import pytest
 
@@ -9,11 +10,14 @@ from gpu_cases import build_product
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize('nx,ny,T,PBC', [(96, 70, 120.0, True), (1, 400, 20.0, False), (200, 3, 60.0, False)])
+@pytest.mark.parametrize('lattice,nx,ny,T,PBC', [
+    ('OOP_Square', 96, 70, 120.0, True), ('OOP_Square', 1, 400, 20.0, False), ('OOP_Square', 200, 3, 60.0, False),
+    ('IP_Kagome', 120, 71, 100.0, False),      # triangles: cells of one layer are neighbours of each other
+])
 @pytest.mark.parametrize('engine', [True, False])
-def test_large_clusters_against_oracle(nx, ny, T, PBC, engine):
+def test_large_clusters_against_oracle(lattice, nx, ny, T, PBC, engine):
     import hotspice_b200 as hs
-    spec = {'lattice': 'OOP_Square', 'a': 200e-9, 'moment': 1e-15, 'nx': nx, 'ny': ny, 'seed': 33, 'kw': {'PBC': PBC},
+    spec = {'lattice': lattice, 'a': 200e-9, 'moment': 1e-15, 'nx': nx, 'ny': ny, 'seed': 33, 'kw': {'PBC': PBC},
             'energies': [{'type': 'exchange', 'J': 1e-21}],
             'params': {'UPDATE_SCHEME': 'Wolff', 'MULTISAMPLING_SCHEME': 'cluster'}}
     fx = {'T': T, 'E_B': np.zeros((ny, nx)), 'm0': np.ones((ny, nx), dtype=int)}
