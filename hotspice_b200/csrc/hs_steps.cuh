@@ -927,6 +927,7 @@ HS_DEV void metro_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
     uint64_t call = C->rng_call;
     if (P.sample_scheme == HS_SAMPLE_GRID && P.n_sc <= 32) {
         __shared__ int s_done;
+        __syncthreads();   // every warp has tested the stop rule before warp 0 writes what it reads
         if (threadIdx.x < 32) {
             const bool d = metro_grid_warp(L, C, sw, P, call);
             if (threadIdx.x == 0) s_done = d;
@@ -1291,6 +1292,7 @@ HS_DEV void wolff_step_cta(const HsLattice &L, HsCounters *C, const HsSwitchList
     }
     const int nx = L.nx, ny = L.ny;
     const int64_t N = (int64_t)nx * ny;
+    __syncthreads();   // every warp has tested the stop rule before warp 0 writes what it reads
     if (threadIdx.x < 32) {
         // seed: _select_single (np.random.randint(n) -> nonzero index)
         const uint64_t c = C->rng_call;
