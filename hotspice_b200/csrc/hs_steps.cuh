@@ -1148,12 +1148,14 @@ struct WolffScratch {
 constexpr int WF_HASH = 512;        // slots: cells checked, with the layer in which they joined
 constexpr int WF_CHECKED = 320;     // cells checked at most (load factor 5/8)
 constexpr int WF_CELLS = 160;       // cells of the cluster at most
+constexpr int WF_MASK = sizeof(HsLattice::nn);   // entries of a neighbour mask at most
+static_assert(WF_MASK <= 32, "a lane per entry");
 struct __align__(16) WolffFast {       // key is cleared in 16-byte words
     int key[WF_HASH];               // flat cell index, -1 empty
     int layer[WF_HASH];             // -1: checked, not a member
     int cell[WF_CELLS], yx[WF_CELLS];
     int cand[WF_CHECKED], cand_yx[WF_CHECKED], cand_slot[WF_CHECKED];
-    int off[25], w[25];             // the neighbour mask's entries: (dy << 16) + dx + 32768, weight
+    int off[WF_MASK], w[WF_MASK];   // the neighbour mask's entries: (dy << 16) + dx + 32768, weight
     int nb;                         // of them
     int lstart, lend, layers, grown; // where a larger cluster goes on; grown: the step is complete
     unsigned long long call;
@@ -1179,7 +1181,7 @@ HS_DEV void wolff_grow_warp(const HsLattice &L, WolffFast &F, int seed, uint64_t
     const unsigned below = (1u << lane) - 1u;
     const int nx = L.nx, ny = L.ny, ch = L.nn_h / 2, cw = L.nn_w / 2;
     for (int k = lane; k < WF_HASH / 4; k += 32) reinterpret_cast<int4 *>(F.key)[k] = make_int4(-1, -1, -1, -1);
-    const int n_mask = L.nn_h * L.nn_w;           // at most 25
+    const int n_mask = L.nn_h * L.nn_w;           // at most WF_MASK
     const int wt = lane < n_mask ? L.nn[lane] : 0;
     const unsigned nz = __ballot_sync(0xffffffffu, wt != 0);
     if (wt) {
@@ -1201,7 +1203,8 @@ HS_DEV void wolff_grow_warp(const HsLattice &L, WolffFast &F, int seed, uint64_t
     }
     __syncwarp();
     auto coord = [](int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); };    // one period off at most
-    const bool odd_size = nx < 3 || ny < 3 || nx > 65535 || ny > 32767;   // wraps twice, or beyond the packing
+    // a neighbour wraps twice, or a coordinate is beyond the packing
+    const bool odd_size = nx < max(3, cw) || ny < max(3, ch) || nx > 65535 || ny > 32767;
     int lstart = 0, lend = 1, checked = 1, layer = 1;
     bool grown = false;
     for (;; ++layer) {
