@@ -1192,7 +1192,7 @@ class Magnets(ABC):
 
     @staticmethod
     def _relax_word(buf, k):
-        """Word k of the relax scratch's header: 0 = stop rule fired, 1 = sweeps made."""
+        """Word k of the relax scratch's header: 0 = stop rule fired (1) or gave up (2), 1 = sweeps made."""
         return int(buf[4 * k:4 * k + 4].cpu().view(torch.int32)[0])
 
     def _replay(self, key, enqueue):
@@ -1264,10 +1264,15 @@ class Magnets(ABC):
                 _lib.check(lib.hs_relax_run(L, C, int(ignore_barrier), n_max, 256, buf.data_ptr(), buf.numel(), st),
                            'hs_relax_run')
                 made += 256
-            if self._relax_word(buf, 0):
+            word = self._relax_word(buf, 0)
+            if word == 2:      # a grid barrier ran out of time: energies of the spins reached, no status left behind
+                self._write_counters(status=self.status & ~_lib.HS_ST_TIMEOUT)
+                self.resync_energies()
+                self.check_resync()
+                raise RuntimeError('relax() gave up: a grid barrier ran out of time (hs_set_wait_limit). The spins are '
+                                   'those reached, with their energies')
+            if word:
                 break
-        if self.status & _lib.HS_ST_TIMEOUT:
-            raise RuntimeError(f'device step reported status {self.status} (HS_ST_* bits)')
         self.relax_sweeps = self._relax_word(buf, 1)
         if verbose:
             print(f"Used {self.relax_sweeps} (out of {n_max}) steps in relax().")

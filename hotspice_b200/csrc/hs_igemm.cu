@@ -33,6 +33,8 @@
 // frees TMEM.
 #include <cuda_bf16.h>
 
+#include <atomic>
+
 #include "hs_common.cuh"
 #include "hs_internal.h"
 
@@ -542,13 +544,14 @@ int64_t hs_igemm_scratch(const HsLattice &L, int nsplit) {
     return layout_of(L, nsplit).total;
 }
 
-// Limit of one pipeline wait of the implicit GEMM (hs_set_wait_limit; WAIT_NS by default).
-static unsigned long long g_wait_ns = WAIT_NS;
+// Limit of one wait inside a kernel (hs_set_wait_limit), 0: the kernel's own (here WAIT_NS).
+static std::atomic<unsigned long long> g_wait_ns{0};
 
 int hs_set_wait_limit_impl(unsigned long long ns) {
-    g_wait_ns = ns ? ns : WAIT_NS;
+    g_wait_ns = ns;
     return HS_OK;
 }
+unsigned long long hs_wait_limit_impl() { return g_wait_ns; }
 
 int hs_launch_igemm(const HsLattice &L, int nsplit, void *scratch, int64_t scratch_bytes, cudaStream_t st) {
     if (nsplit < 1 || nsplit > MAX_SPLIT) { hs_set_error("hs_dipolar_full_igemm: nsplit must be 1..3"); return HS_EINVAL; }
@@ -585,6 +588,7 @@ int hs_launch_igemm(const HsLattice &L, int nsplit, void *scratch, int64_t scrat
     cudaError_t e = cudaFuncSetAttribute(igemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) { hs_set_error("igemm smem attribute: %s", cudaGetErrorString(e)); return HS_ECUDA; }
 
+    const unsigned long long wait_ns = hs_wait_limit_impl() ? hs_wait_limit_impl() : WAIT_NS;
     const int grid = lo.XT * lo.YT * lo.KS;
     for (int pass = 0; pass < (L.use_perp ? 2 : 1); ++pass) {
         double *out = pass == 0 ? L.E_dip : L.E_dip_perp;
@@ -596,7 +600,7 @@ int hs_launch_igemm(const HsLattice &L, int nsplit, void *scratch, int64_t scrat
         cudaMemsetAsync(out, 0, sizeof(double) * (size_t)L.nx * L.ny, st);
         for (int s = 0; s < L.n_sub; ++s) {
             IgemmParams p{strips, spins, lo.qspan, lo.qmin, nsplit, s, lo.P, lo.C, L.nx, L.ny, lo.rows, lo.XT, lo.KS, lo.G, acc, status,
-                          g_wait_ns};
+                          wait_ns};
             igemm_kernel<<<grid, NT, SMEM_BYTES, st>>>(p);
             if ((rc = hs_check_launch("igemm_kernel"))) return rc;
             igemm_finalize_kernel<<<148 * 4, 256, 0, st>>>(acc, lo.KS, lo.P, L.nx, L.ny, L.ux, L.uy, L.sub_of, s, L.m, L.moment,

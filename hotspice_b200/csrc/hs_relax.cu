@@ -38,13 +38,14 @@ constexpr int RX_PER = 4;               // candidates per thread
 constexpr int RX_CH = RX_T * RX_PER;    // candidates per block
 constexpr int RX_MAX_P = 1024;          // subgrids per sweep (4 * 256 unit-cell sites)
 constexpr int RX_MAX_U = 256;           // unit-cell sites
+constexpr int RX_GAVE_UP = 2;           // RelaxState::done after a grid barrier that ran out of time
 constexpr int MN_PASSES = 5;            // radix-select passes over the 53-bit keys
 constexpr int MN_BINS = 2048;           // largest digit (11 bits)
 __constant__ int c_mn_lo[MN_PASSES] = {42, 31, 20, 10, 0};
 __constant__ int c_mn_bits[MN_PASSES] = {11, 11, 11, 10, 10};
 
 struct RelaxState {
-    int32_t done;       // stop rule fired: the remaining kernels of the sweep do nothing
+    int32_t done;       // stop rule fired (or RX_GAVE_UP): the remaining kernels of the sweep do nothing
     int32_t sweep;      // sweeps completed (relax)
     int32_t differs;    // the state after this sweep differs from the one two sweeps before
     int32_t pad0;
@@ -284,19 +285,26 @@ struct RelaxGrid {          // zeroed before every launch
 struct RelaxPlan {
     int sx, sy, TX, TY, tiles_x, tiles, words, rows;   // words per bitmap row, rows of the largest subgrid
     int ignore_barrier, n_max, max_sweeps;
-    unsigned long long wait_ns;
+    unsigned poll_mask;                 // a waiting CTA looks at the time and at `abort` every poll_mask + 1 polls
+    unsigned long long wait_ns;         // limit of one barrier
     unsigned *bits;         // [2][rows][words]
     RelaxGrid *g;
 };
 
-constexpr unsigned long long RX_WAIT_NS = 4000000000ULL;   // a grid barrier gives up after 4 s
+// Limit of a grid barrier: hs_set_wait_limit's when one is set, else 4 s more than the longest time
+// between two barriers of one CTA. That time is bounded by the switches in reach of a warp's cells
+// times the warp's parts; a switch takes a warp 0.3 us (512 x 512 pinwheel, 160 in reach: 96 K cycles
+// for the update of a crowded subgrid), several times that with truncated periodic windows.
+constexpr unsigned long long RX_WAIT_NS = 4000000000ULL;
+constexpr double RX_SWITCH_NS = 4000.0;
 
 // Grid barrier number `k` (0, 1, ...) of this launch, adding up every CTA's `v`: the sum of this
 // barrier's, or -1 when it gave up (then on every CTA, sooner or later). `seen` keeps the two words'
 // earlier sums. A CTA still polling a word never meets later arrivals: those of barrier k + 1 go to
 // the other word, and those of k + 2 wait for it at k + 1.
-HS_DEV int grid_barrier(RelaxGrid *g, unsigned k, unsigned v, unsigned (&seen)[2], unsigned long long limit_ns) {
+HS_DEV int grid_barrier(const RelaxPlan &P, unsigned k, unsigned v, unsigned (&seen)[2]) {
     __shared__ int s_sum;
+    RelaxGrid *const g = P.g;
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long *word = &g->bar[k & 1];
@@ -309,9 +317,9 @@ HS_DEV int grid_barrier(RelaxGrid *g, unsigned k, unsigned v, unsigned (&seen)[2
             unsigned long long w;
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(word) : "memory");
             if ((unsigned)w >= want) { sum = (int)((unsigned)(w >> 32) - seen[k & 1]); break; }
-            if ((it & 255) == 255) {
+            if ((it & P.poll_mask) == P.poll_mask) {
                 if (*(volatile int *)&g->abort) break;
-                if (hs_globaltimer_ns() - t0 > limit_ns) { atomicExch(&g->abort, 1); break; }
+                if (hs_globaltimer_ns() - t0 > P.wait_ns) { atomicExch(&g->abort, 1); break; }
             }
         }
         s_sum = sum;
@@ -561,7 +569,7 @@ __global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCoun
     if (B.st->done) return;
     int sweep = B.st->sweep, done = 0;
     const uint64_t call0 = C->rng_call;
-    long long switched = 0;              // by this launch (every CTA counts)
+    long long switched = 0, sweep_total = 0;   // by this launch and by the sweep (every CTA counts)
     unsigned nbar = 0, slot = 0;         // barriers passed, subgrids so far
     unsigned seen[2] = {0u, 0u};
     int made = 0;
@@ -577,7 +585,7 @@ __global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCoun
             s_order[rank] = e;
         }
         __syncthreads();
-        long long sweep_total = 0;
+        sweep_total = 0;
         for (int i = 0; i < n_sub && ok; ++i) {
             const int o = s_order[i];
             const int y0 = o / P.sx, x0 = o % P.sx;
@@ -615,7 +623,7 @@ __global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCoun
                 }
             }
             mine = block_sum(lane == 0 ? mine : 0, s_w);
-            const int all = grid_barrier(P.g, nbar++, (unsigned)mine, seen, P.wait_ns);
+            const int all = grid_barrier(P, nbar++, (unsigned)mine, seen);
             ok = all >= 0;
             if (L.has_exchange && ok) {
                 for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
@@ -629,7 +637,7 @@ __global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCoun
                             L.mm[c] = -L.mm[c];
                         }
                 }
-                ok = grid_barrier(P.g, nbar++, 0u, seen, P.wait_ns) >= 0;
+                ok = grid_barrier(P, nbar++, 0u, seen) >= 0;
             }
             if (!ok) break;
             sweep_total += all;
@@ -654,8 +662,8 @@ __global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCoun
             }
             ++slot;
         }
-        if (!ok) break;
         switched += sweep_total;
+        if (!ok) break;
         // the stop rule (relax_compare_kernel, relax_end_kernel)
         if (sweep_total == 0) { done = 1; ++sweep; continue; }
         int8_t *snap = B.snap + ((sweep + 1) & 1) * N;
@@ -671,7 +679,7 @@ __global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCoun
             }
         }
         d = block_sum(d, s_w);
-        const int differs = grid_barrier(P.g, nbar++, d ? 1u : 0u, seen, P.wait_ns);
+        const int differs = grid_barrier(P, nbar++, d ? 1u : 0u, seen);
         ok = differs >= 0;
         if (!ok) break;
         ++sweep;
@@ -684,7 +692,7 @@ __global__ void __launch_bounds__(RX_T, 1) relax_grid_kernel(HsLattice L, HsCoun
         C->switches += switched;
         C->attempted += switched;
         C->n_sw = 0;
-        if (!ok) { C->status |= HS_ST_TIMEOUT; B.st->done = 1; }
+        if (!ok) { C->status |= HS_ST_TIMEOUT; B.st->done = RX_GAVE_UP; }
     }
 }
 
@@ -1110,7 +1118,9 @@ int hs_relax_run_impl(const HsLattice &L, HsCounters *C, int ignore_barrier, int
     P.ignore_barrier = ignore_barrier;
     P.n_max = n_max;
     P.max_sweeps = max_sweeps;
-    P.wait_ns = RX_WAIT_NS;
+    const unsigned long long limit = hs_wait_limit_impl();
+    P.wait_ns = limit;
+    P.poll_mask = limit && limit < 1000000ULL ? 0u : 255u;
     P.bits = reinterpret_cast<unsigned *>(B.cells);       // at most 4 N bytes: minimize()'s list
     P.g = reinterpret_cast<RelaxGrid *>(B.hist);
     static_assert(sizeof(RelaxGrid) <= 4 * MN_PASSES * MN_BINS, "the grid state lives in minimize()'s histograms");
@@ -1120,6 +1130,13 @@ int hs_relax_run_impl(const HsLattice &L, HsCounters *C, int ignore_barrier, int
     HsLattice Lv = L;
     void *args[] = {&Lv, &C, &B, &P};
     const int grid = std::max(1, std::min(P.tiles, sms * std::max(per, 1)));
+    if (!limit) {
+        const int hy = L.trunc_size ? std::max(L.dip_wy, std::min(L.trunc_size, L.ny - 1)) : L.ny - 1;
+        const int hx = L.trunc_size ? std::max(L.dip_wx, std::min(L.trunc_size, L.nx - 1)) : L.nx - 1;
+        const double reach = (std::min(L.ny, 2 * hy + RX_V) / P.sy + 1.0) * (std::min(L.nx, 2 * hx + 32) / P.sx + 1.0);
+        const double parts = std::ceil(P.sx * std::ceil((double)P.TY / RX_V) / (RX_T / 32)) * ((P.tiles + grid - 1) / grid);
+        P.wait_ns = RX_WAIT_NS + (unsigned long long)(reach * parts * RX_SWITCH_NS);
+    }
     e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(relax_grid_kernel), dim3(grid), dim3(RX_T), args,
                                     sizeof(RelaxShared), st);
     if (e != cudaSuccess) { hs_set_error("relax_grid_kernel: %s", cudaGetErrorString(e)); return HS_ECUDA; }

@@ -229,10 +229,12 @@ int hs_dipolar_full_fft(const HsLattice *L, void *scratch, int64_t scratch_bytes
 int64_t hs_igemm_scratch_bytes(const HsLattice *L, int32_t nsplit);
 int hs_dipolar_full_igemm(const HsLattice *L, int32_t nsplit, void *scratch, int64_t scratch_bytes, void *stream);
 
-/* Limit, in ns of wall time, of one pipeline wait inside hs_dipolar_full_igemm (0: the default,
- * 4 s). A wait that runs out sets bit 0 of the call's status word and the kernel ends cleanly (its
- * copies land, its MMAs finish, TMEM is freed). No reference counterpart: a safety bound of this
- * library, shortened only to test that path. Applies to later calls of this process. */
+/* Limit, in ns of wall time, of one wait inside a kernel (0: the kernel's own): of a pipeline wait of
+ * hs_dipolar_full_igemm (4 s) and of a grid barrier of hs_relax_run (4 s more than the work between
+ * two barriers can take). A wait that runs out ends its kernel cleanly: hs_dipolar_full_igemm sets
+ * bit 0 of the call's status word (its copies land, its MMAs finish, TMEM is freed), hs_relax_run
+ * sets HS_ST_TIMEOUT. No reference counterpart: a safety bound of this library, shortened only to
+ * test that path. Applies to later calls of this process. */
 int hs_set_wait_limit(uint64_t ns);
 
 /* ---- (c) Néel-Arrhenius step ------------------------------------------------------------- */
@@ -285,7 +287,10 @@ int hs_relax_check(const HsLattice *L, HsCounters *C, int32_t n_max, void *scrat
                    void *stream);
 /* Up to max_sweeps sweeps (not simultaneous) with hs_relax_check's stop rule after each, in one
  * cooperative launch; the same state as that many hs_minimize_all / hs_relax_check pairs, except that
- * n_sw is 0 afterwards. Needs the whole launch resident at once (it waits for the GPU otherwise). */
+ * n_sw is 0 afterwards. Needs the whole launch resident at once (it waits for the GPU otherwise).
+ * When a grid barrier runs out of time (hs_set_wait_limit) it sets HS_ST_TIMEOUT and leaves 2 in the
+ * first word of the scratch (1: the stop rule fired); spins and moments are then those reached, the
+ * dipolar energies have to be recomputed. */
 int hs_relax_run(const HsLattice *L, HsCounters *C, int32_t ignore_barrier, int32_t n_max, int32_t max_sweeps,
                  void *scratch, int64_t scratch_bytes, void *stream);
 /* Start minimize(): clears the stop state and the per-magnet pick counts. */
