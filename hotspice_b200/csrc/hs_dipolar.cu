@@ -534,7 +534,7 @@ dip_update_few_kernel(HsLattice L, HsSwitchList sw, const int32_t *n_sw_dev, int
     const int nsw = min(n_sw_dev ? *n_sw_dev : n_host, cap);
     if (nsw <= 0) return;
     const int n_items = few_stage<FEW_R>(L, w, nsw, semantics, s_sw, s_w);
-    few_items<FEW_R>(L, s_sw, nsw, n_items, semantics, blockIdx.x * (FEW_T / 32) + (threadIdx.x >> 5), gridDim.x * (FEW_T / 32));
+    few_items_of<FEW_R, false>(L, s_sw, nsw, n_items, semantics, blockIdx.x * (FEW_T / 32) + (threadIdx.x >> 5), gridDim.x * (FEW_T / 32));
 }
 
 // Direct-sum full recompute, one thread per target cell (hotspice/energies.py:290-308):
@@ -601,7 +601,8 @@ int hs_launch_dipolar_update(const HsLattice &L, const HsSwitchList &sw, const i
     const int64_t items = (int64_t)((std::min(2 * hy + 1, L.ny) + FEW_R - 1) / FEW_R) * ((std::min(2 * hx + 1, L.nx) + 31) / 32);
     // Short lists with windows of up to about 128 x 256 cells: the work follows the switches. With
     // longer lists every item looks for windows it meets among too many (625 windows of 79 x 79: 91 us
-    // against 44 us of the persistent kernel), with uncut windows every switch visits the lattice.
+    // against 44 us of the persistent kernel). Uncut windows were measured when every switch still
+    // visited the whole lattice (Poisson, 1024 x 1024: 162 against 17 us) and stay with those kernels.
     if (most <= FEW_MAX && items <= FEW_ITEMS) {
         const int cap = std::max(most, 1);
         const int grid = (int)std::min<int64_t>(2 * 148, (cap * items + FEW_T / 32 - 1) / (FEW_T / 32));

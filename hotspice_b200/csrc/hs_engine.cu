@@ -1000,6 +1000,10 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
             S.all();
             if (L.has_dipolar) {
                 const int nsw = sh.nsw;
+                // Short lists go by their windows, whatever their size. Us per step on 1 / 16 CTAs, beside
+                // the longer lists' code: 512 x 512, cutoff 20a, 5 switches 13.7 / 8.2 (32.5 / 10.7);
+                // 256 x 256 uncut, 21 switches 103 / 18.6 (299 / 51.8); 1024 x 1024 uncut, 22 switches
+                // 1472 / 123 (2050 / 174).
                 if (nsw > 0 && nsw <= FEW_MAX) {       // uniform over the instance's threads
                     FewSw w{};
                     if ((int)threadIdx.x < nsw) {

@@ -69,7 +69,9 @@ HS_DEV void hs_contrib(const HsLattice &L, const SwInfo &w, int y, int x, float 
 // for bit. The common item meets no other window and reads nothing but its own cells and kernel rows.
 // Measured on B200 (cutoff 20a, 79 x 79 windows): us per step of two kernels, 512 x 512
 // 7.7 -> 6.7 and 1500 x 1201 with about 20 switches 18.6 -> 10.8; bound by the latencies of list,
-// moments, cells and the two launches.
+// moments, cells and the two launches. Where the windows add up to more than the lattice
+// (few_crowded), one inside an earlier one gets no items: with uncut windows a cell is visited once,
+// not once per switch.
 constexpr int FEW_MAX = 64, FEW_ITEMS = 128;
 
 struct FewSw {
@@ -80,9 +82,35 @@ struct FewSw {
     int end;                 // items of the switches up to this one
 };
 
+// hs_minimage of the difference of two coordinates, without the remainder.
+HS_DEV int few_minimage(int d, int n) {
+    d = d < 0 ? d + n : d;
+    return 2 * d >= n ? d - n : d;
+}
+
 HS_DEV bool few_covers(const HsLattice &L, const FewSw &w, int y, int x) {
-    if (w.kind == 0) return abs(y - w.y) <= w.hy && abs(x - w.x) <= w.hx;
-    return hs_axis_overlap(w.y, w.hy, 1, L.ny, y, 1) && hs_axis_overlap(w.x, w.hx, 1, L.nx, x, 1);
+    int dy = y - w.y, dx = x - w.x;
+    if (w.kind) { dy = few_minimage(dy, L.ny); dx = few_minimage(dx, L.nx); }
+    return abs(dy) <= w.hy && abs(dx) <= w.hx;
+}
+
+// Are all of coordinates t0 .. t0 + tn - 1 (not reduced to 0 .. n - 1 where windows wrap) within `half` of s?
+HS_DEV bool few_axis_inside(int s, int half, bool wrap, int n, int t0, int tn) {
+    if (!wrap) return t0 >= s - half && t0 + tn - 1 <= s + half;
+    return 2 * half + 1 >= n || hs_wrap(t0 - (s - half), n) + tn <= 2 * half + 1;
+}
+
+// Does the window of w, which comes earlier in the list, hold all of the rectangle (`wraps`: it may
+// reach beyond the lattice)? Its cells are w's then, or an even earlier window's.
+HS_DEV bool few_holds(const HsLattice &L, const FewSw &w, int semantics, bool wraps, int y0, int nr, int x0, int nc) {
+    if ((w.sub < 0 && semantics != HS_UPDATE_MULTIPLE) || (wraps && w.kind == 0)) return false;
+    return few_axis_inside(w.y, w.hy, w.kind != 0, L.ny, y0, nr) && few_axis_inside(w.x, w.hx, w.kind != 0, L.nx, x0, nc);
+}
+
+// Do the windows add up to more than the lattice, so that many of them lie in earlier ones?
+template <int R>
+HS_DEV bool few_crowded(const HsLattice &L, int nsw, int n_items) {
+    return nsw > 1 && (int64_t)n_items * (32 * R) > (int64_t)L.nx * L.ny;
 }
 
 // Stage switch k (w.y, w.x, w.mode loaded by thread k < nsw) and number the items through; returns
@@ -112,22 +140,34 @@ HS_DEV int few_stage(const HsLattice &L, FewSw w, int nsw, int semantics, FewSw 
         if (w.sub >= 0 || semantics == HS_UPDATE_MULTIPLE)
             items = ((w.nr + R - 1) / R) * ((w.nc + 31) / 32);
     }
-    int incl = items;
+    auto number = [&]() {
+        int incl = items, before = 0, total = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
-    if (lane == 31 && warp < FEW_MAX / 32) s_w[warp] = incl;
-    __syncthreads();
-    int before = 0, n_items = 0;
+        for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+        if (lane == 31 && warp < FEW_MAX / 32) s_w[warp] = incl;
+        __syncthreads();
 #pragma unroll
-    for (int q = 0; q < FEW_MAX / 32; ++q) { if (q < warp) before += s_w[q]; n_items += s_w[q]; }
-    if (k < nsw) { w.end = before + incl; s_sw[k] = w; }
-    __syncthreads();
+        for (int q = 0; q < FEW_MAX / 32; ++q) { if (q < warp) before += s_w[q]; total += s_w[q]; }
+        if (k < nsw) { w.end = before + incl; s_sw[k] = w; }
+        __syncthreads();
+        return total;
+    };
+    int n_items = number();
+    if (few_crowded<R>(L, nsw, n_items)) {       // uniform; windows inside an earlier one need no items
+        if (k < nsw)
+            for (int q = 0; q < k && items; ++q)
+                if (few_holds(L, s_sw[q], semantics, w.kind != 0, w.ylo, w.nr, w.xlo, w.nc)) items = 0;
+        __syncthreads();
+        n_items = number();
+    }
     return n_items;
 }
 
-// The items gw, gw + nw, ... of a staged list; a warp calls it.
-template <int R>
-HS_DEV void few_items(const HsLattice &L, const FewSw *s_sw, int nsw, int n_items, int semantics, int gw, int nw) {
+// The items gw, gw + nw, ... of a staged list; a warp calls it. CROWDED: an item inside an earlier
+// window leaves before it loads anything, and one whose cells all belong to earlier windows before it
+// adds the later ones. Without overlaps these tests cost 5%, so they are compiled apart.
+template <int R, bool CROWDED>
+HS_DEV void few_items_of(const HsLattice &L, const FewSw *s_sw, int nsw, int n_items, int semantics, int gw, int nw) {
     const int lane = threadIdx.x & 31, nx = L.nx, ny = L.ny;
     const bool two = L.use_perp != 0, flip_perp = !(L.dip_keep_perp_sign && nsw > 1);
     const float pref2 = (float)(2.0 * L.dip_pref);
@@ -143,6 +183,12 @@ HS_DEV void few_items(const HsLattice &L, const FewSw *s_sw, int nsw, int n_item
         const int tr = tile / tc_n, tc = tile - tr * tc_n;
         const int y0 = own.ylo + R * tr, x0 = own.xlo + 32 * tc, nr = min(R, own.nr - R * tr);
         const int ncol = min(32, own.nc - 32 * tc);
+        const bool wraps = y0 < 0 || y0 + nr > ny || x0 < 0 || x0 + ncol > nx;
+        if constexpr (CROWDED) {           // leave before any load when an earlier window holds the item
+            bool held = false;
+            for (int b = lane; b < k; b += 32) held |= few_holds(L, s_sw[b], semantics, wraps, y0, nr, x0, ncol);
+            if (__any_sync(0xffffffffu, held)) continue;
+        }
         int x = x0 + lane;
         const bool inx = lane < ncol;
         x = x < 0 ? x + nx : (x >= nx ? x - nx : x);
@@ -163,10 +209,11 @@ HS_DEV void few_items(const HsLattice &L, const FewSw *s_sw, int nsw, int n_item
         }
         float acc[R] = {}, accp[R] = {};
         unsigned mine = inx ? (1u << nr) - 1u : 0u, neg = 0u;
-        auto apply = [&](const FewSw &w, bool all_in) {
-            const int dx0 = x - w.x;
-            if (w.kind == 0 && all_in) {   // the item's own plain window: every cell lies in it
-                const float *K = Kg + ((int64_t)max(w.sub, 0) * KH + (row[0] - w.y + L.dip_wy)) * KW + (dx0 + L.dip_wx);
+        auto apply = [&](const FewSw &w, bool item_own) {
+            int dx = x - w.x;
+            const bool own_col = dx == 0;
+            if (w.kind == 0 && item_own) {   // the item's own plain window: every cell lies in it
+                const float *K = Kg + ((int64_t)max(w.sub, 0) * KH + (row[0] - w.y + L.dip_wy)) * KW + (dx + L.dip_wx);
                 const float *Kp = two ? Kpg + (K - Kg) : nullptr;
                 float kv[R], kp[R];
 #pragma unroll
@@ -174,32 +221,51 @@ HS_DEV void few_items(const HsLattice &L, const FewSw *s_sw, int nsw, int n_item
                     const bool in = inx && v < nr && w.sub >= 0;
                     kv[v] = in ? __ldg(K + v * KW) : 0.f;
                     kp[v] = in && two ? __ldg(Kp + v * KW) : 0.f;
-                    if (dx0 == 0 && row[v] == w.y) neg |= 1u << v;
+                    if (own_col && row[v] == w.y) neg |= 1u << v;
                 }
 #pragma unroll
                 for (int v = 0; v < R; ++v) { acc[v] += w.mm * kv[v]; accp[v] += w.mm * kp[v]; }
                 return;
             }
+            if (w.kind == 2) {
+#pragma unroll
+                for (int v = 0; v < R; ++v) {
+                    if (!inx || v >= nr || !(item_own || few_covers(L, w, row[v], x))) continue;
+                    if (own_col && row[v] == w.y) neg |= 1u << v;
+                    if (w.sub >= 0) hs_contrib(L, SwInfo{w.y, w.x, w.mode, w.sub, w.mm}, row[v], x, acc[v], accp[v]);
+                }
+                return;
+            }
+            // no branch per cell, so that the loads of all rows are in flight together
+            if (w.kind) dx = few_minimage(dx, nx);
+            const float *K = Kg + ((int64_t)max(w.sub, 0) * KH + L.dip_wy) * KW + (L.dip_wx + dx);
+            const float *Kp = two ? Kpg + (K - Kg) : nullptr;
+            float kv[R], kp[R];
+            bool in[R];
+            const bool in_col = inx && abs(dx) <= w.hx;
 #pragma unroll
             for (int v = 0; v < R; ++v) {
-                if (!inx || v >= nr || !(all_in || few_covers(L, w, row[v], x))) continue;
-                if (dx0 == 0 && row[v] == w.y) neg |= 1u << v;
-                if (w.sub < 0) continue;
-                if (w.kind == 2) { hs_contrib(L, SwInfo{w.y, w.x, w.mode, w.sub, w.mm}, row[v], x, acc[v], accp[v]); continue; }
-                acc[v] += w.mm * hs_kval(L, Kg, w.sub, row[v] - w.y, dx0);
-                if (two) accp[v] += w.mm * hs_kval(L, Kpg, w.sub, row[v] - w.y, dx0);
+                int dy = row[v] - w.y;
+                if (w.kind) dy = few_minimage(dy, ny);
+                in[v] = in_col && v < nr && abs(dy) <= w.hy;
+                if (in[v] && own_col && row[v] == w.y) neg |= 1u << v;
+                in[v] = in[v] && w.sub >= 0;
+                kv[v] = in[v] ? __ldg(K + dy * KW) : 0.f;
+                kp[v] = in[v] && two ? __ldg(Kp + dy * KW) : 0.f;
             }
+#pragma unroll
+            for (int v = 0; v < R; ++v) if (in[v]) { acc[v] += w.mm * kv[v]; accp[v] += w.mm * kp[v]; }
         };
         // windows that may meet the item, in list order
-        const bool wraps = y0 < 0 || y0 + nr > ny || x0 < 0 || x0 + ncol > nx;
-        for (int b = 0; b < nsw; b += 32) {
+        bool live = true;                  // warp-uniform: some cell is not an earlier window's (CROWDED)
+        for (int b = 0; b < nsw && live; b += 32) {
             bool meets = false;
             if (b + lane < nsw) {
                 const FewSw &w = s_sw[b + lane];
                 meets = b + lane == k || wraps ||
                         (hs_axis_overlap(w.y, w.hy, w.kind != 0, ny, y0, nr) && hs_axis_overlap(w.x, w.hx, w.kind != 0, nx, x0, ncol));
             }
-            for (unsigned m = __ballot_sync(0xffffffffu, meets); m; m &= m - 1u) {
+            for (unsigned m = __ballot_sync(0xffffffffu, meets); m && live; m &= m - 1u) {
                 const int q = b + __ffs(m) - 1;
                 if (q == k) { apply(own, true); continue; }
                 const FewSw w = s_sw[q];
@@ -208,6 +274,7 @@ HS_DEV void few_items(const HsLattice &L, const FewSw *s_sw, int nsw, int n_item
 #pragma unroll
                 for (int v = 0; v < R; ++v)
                     if (((mine >> v) & 1u) && few_covers(L, w, row[v], x)) mine &= ~(1u << v);   // an earlier window's cell
+                if constexpr (CROWDED) live = __any_sync(0xffffffffu, mine != 0u);
             }
         }
 #pragma unroll
@@ -228,6 +295,12 @@ HS_DEV void few_items(const HsLattice &L, const FewSw *s_sw, int nsw, int n_item
             if (two) Epg[i] = p;
         }
     }
+}
+
+template <int R>
+HS_DEV void few_items(const HsLattice &L, const FewSw *s_sw, int nsw, int n_items, int semantics, int gw, int nw) {
+    if (few_crowded<R>(L, nsw, n_items)) few_items_of<R, true>(L, s_sw, nsw, n_items, semantics, gw, nw);
+    else few_items_of<R, false>(L, s_sw, nsw, n_items, semantics, gw, nw);
 }
 
 // ---- Metropolis ------------------------------------------------------------------------

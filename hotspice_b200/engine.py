@@ -57,8 +57,10 @@ def step_model(mm: Magnets) -> tuple[float, float, float]:
     class (dense / half / sparse, which also carries the perpendicular channel of the in-plane
     lattices), Néel steps spread over the cluster like cs^0.85 (512 x 512 dense: 172 us on one CTA,
     16.5 us on 16; 64 x 64: 7.4 and 5.1 us) and Metropolis steps like cs^0.5; a Wolff step grows its
-    cluster on one CTA and costs about 6 us above the critical temperature. Inside a full batch the
-    CTAs share the L2, so a batch's launch plan is best measured (:meth:`BatchEngine.tune_split`)."""
+    cluster on one CTA and costs about 6 us above the critical temperature. The Metropolis figures
+    are those of a cutoff of 16 lattice constants; a larger window costs in proportion (1024 x 1024
+    uncut, 22 switches a step: 1.5 ms on one CTA, 0.12 ms on 16). Inside a full batch the CTAs share the L2, so a
+    batch's launch plan is best measured (:meth:`BatchEngine.tune_split`)."""
     n = mm.nx * mm.ny
     f = mm.n / max(n, 1)
     cls = 0 if f >= 0.75 else (1 if f >= 0.45 else 2)
@@ -69,7 +71,14 @@ def step_model(mm: Magnets) -> tuple[float, float, float]:
     if sch == Scheme.WOLFF:
         return 5.2 + 6e-6 * n, 0.0, 0.0
     c, beta = ((0.00132, 0.65), (0.0010, 0.75), (0.0009, 0.82))[cls]
-    return 4.0, c * n ** beta, 0.5
+    part = c * n ** beta
+    dipolar = getattr(mm, '_dipolar', None)        # a stand-in made from a request's spec has none
+    d = dipolar() if dipolar else None
+    if d is not None:
+        cells = [min(wy, mm.ny) * min(wx, mm.nx) for wy, wx in
+                 (((33, 33), (65, 65), (73, 129))[cls], (2 * d.kernel_set.wy + 1, 2 * d.kernel_set.wx + 1))]
+        part *= max(1.0, cells[1] / cells[0])
+    return 4.0, part, 0.5
 
 
 def model_time(m, cs):
