@@ -49,8 +49,8 @@ constexpr int UPD_LOC = 2048;                      // staged switches per pass
 template <int VEC>
 __global__ void __launch_bounds__(32 * UPD_WARPS, HS_UPD_MIN_CTAS)
 dip_update_kernel(HsLattice L, HsSwitchList sw, const int32_t *n_sw_dev, int n_host, int semantics,
-                  const HsCounters *C) {
-    hs_pdl_begin();
+                  const HsCounters *C, int overlap) {
+    if (overlap) hs_pdl_begin();
     if (C && C->done) return;
     const int nsw = n_sw_dev ? *n_sw_dev : n_host;
     if (nsw <= 0) return;
@@ -262,7 +262,6 @@ template <int VEC>
 __global__ void __launch_bounds__(32 * UPD_WARPS, HS_UPD_MIN_CTAS)
 dip_update_persist_kernel(HsLattice L, HsSwitchList sw, const int32_t *n_sw_dev, int n_host, int semantics,
                           const HsCounters *C, int tiles, int cap) {
-    hs_pdl_begin();
     if (C && C->done) return;
     const int nsw = n_sw_dev ? *n_sw_dev : n_host;
     if (nsw <= 0 || nsw > cap) return;   // the launcher sends longer lists to dip_update_kernel
@@ -579,8 +578,9 @@ int launch_persist(const HsLattice &L, const HsSwitchList &sw, const int32_t *n_
         if (e != cudaSuccess) { hs_set_error("dip_update_persist_kernel: %s", cudaGetErrorString(e)); return HS_ECUDA; }
         granted = smem;
     }
-    return hs_launch_step("dip_update_persist_kernel", dip_update_persist_kernel<VEC>, persist_grid<VEC>(tiles, smem), 32 * UPD_WARPS,
-                          (size_t)smem, st, L, sw, n_sw_dev, n_host, semantics, C, tiles, cap);
+    dip_update_persist_kernel<VEC><<<persist_grid<VEC>(tiles, smem), 32 * UPD_WARPS, (size_t)smem, st>>>(
+        L, sw, n_sw_dev, n_host, semantics, C, tiles, cap);
+    return hs_check_launch("dip_update_persist_kernel");
 }
 }  // namespace
 
@@ -614,8 +614,16 @@ int hs_launch_dipolar_update(const HsLattice &L, const HsSwitchList &sw, const i
         return vec ? launch_persist<4>(L, sw, n_sw_dev, n_host, semantics, C, tiles, cap, st)
                    : launch_persist<1>(L, sw, n_sw_dev, n_host, semantics, C, tiles, cap, st);
     }
-    return hs_launch_step("dip_update_kernel", vec ? dip_update_kernel<4> : dip_update_kernel<1>, tiles, 32 * UPD_WARPS, 0, st, L, sw,
-                          n_sw_dev, n_host, semantics, C);
+    // Of the long lists' kernels only small launches overlap the kernel before them (256 x 256, 32 tiles:
+    // 12.7 -> 12.5 us per step): with more CTAs that costs more than it hides (per step, plain launch
+    // and overlapped: 512 x 512 uncut 16.4 and 20.4 us, 1000 x 1000 with 570 switches, the persistent
+    // kernel, 75 and 88, 2500 x 2500 with 3000 switches 238 and 279).
+    if (tiles <= 64)
+        return hs_launch_step("dip_update_kernel", vec ? dip_update_kernel<4> : dip_update_kernel<1>, tiles, 32 * UPD_WARPS, 0, st,
+                              L, sw, n_sw_dev, n_host, semantics, C, 1);
+    if (vec) dip_update_kernel<4><<<tiles, 32 * UPD_WARPS, 0, st>>>(L, sw, n_sw_dev, n_host, semantics, C, 0);
+    else dip_update_kernel<1><<<tiles, 32 * UPD_WARPS, 0, st>>>(L, sw, n_sw_dev, n_host, semantics, C, 0);
+    return hs_check_launch("dip_update_kernel");
 }
 
 int hs_launch_dipolar_full_direct(const HsLattice &L, int fp64, double *E64, double *Ep64, cudaStream_t st) {

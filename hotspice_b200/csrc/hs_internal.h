@@ -74,7 +74,8 @@ int hs_engine_max_clusters_impl(int cluster_size);
 // Launch with programmatic stream serialisation: the kernel may start while the one before it in the
 // stream still runs, if that one allows it (hs_pdl_begin's trigger), and must not touch global memory
 // before hs_pdl_begin, which waits until everything before it has finished and is visible. Used for
-// the kernels of a step, whose launch latencies are comparable to their run times.
+// the kernels of a step whose launch latencies are comparable to their run times; a kernel launched
+// without it ends the chain, whether or not its neighbours use it.
 template <typename... P, typename... A>
 int hs_launch_step(const char *what, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A &&...args) {
     cudaLaunchConfig_t cfg = {};
