@@ -495,9 +495,10 @@ class Server:
         prev_end = None          # end event of the last finished round
 
         def collect():
-            """Turn the read-outs that have landed into results."""
+            """Turn the read-outs that have landed into results; whether any has."""
             if not retiring:
-                return
+                return False
+            held = len(retiring)
             now = time.perf_counter()
             still = []
             for a, sm in retiring:
@@ -507,6 +508,7 @@ class Server:
                 else:
                     still.append((a, sm))
             retiring[:] = still
+            return len(still) < held
 
         def build(r):
             # runs on the builder thread: its own stream, an event the rounds wait on
@@ -559,7 +561,8 @@ class Server:
 
         while pending or dealing() or queue or active or inflight or building or retiring:
             admit()
-            collect()
+            if collect() and queue:
+                continue       # what the read-outs held is free for the waiting requests
             runnable = [a for a in active if a.remaining > 0]
             if runnable and len(inflight) < self.max_inflight:
                 # short rounds while requests still arrive (they join at round boundaries),
