@@ -141,6 +141,23 @@ class RunSummary:
                     state=h['state'].numpy().copy() if 'state' in h else None)
 
 
+def fft_is_faster(cells: int, magnets: int, window: int, slots: int, wrap: bool) -> bool:
+    """Is the full sum faster as a convolution (``slots`` complex kernels) than as a direct sum over
+    windows of ``window`` cells? Both sides as modelled from 540 recomputes on B200 (ten lattices, 10 to
+    1000 cells a side, windows of 25 cells to the whole lattice). The direct sum walks a window
+    serially, 0.19 us per entry (0.25 with minimum images), until the GPU is full; the convolution has
+    three launches of a few us each and transforms each slot's kernels: 5 x 5 windows of 200 x 200
+    cells 12 against 40 us, kagome 13 x 7 22 against 67, square 13 x 13 38 against 39, uncut 24 x 24
+    101 against 28. Where it decides wrongly among those, it loses at most 16% (5 us). Up to 9 x 9 the
+    direct sum is taken throughout."""
+    if window <= 81:
+        return False
+    load = (0.7 + 0.3 * magnets / cells) * cells * window
+    direct = max(3 + (0.25 if wrap else 0.19) * window + 5e-7 * load, 15 + 1.6e-6 * load)
+    fft = 22 + min(10, cells / 1000) + 5e-5 * cells + slots * (3 + min(2.5, cells / 5000) + 2e-5 * max(0, cells - 250000))
+    return fft < direct
+
+
 class Magnets(ABC):
     """hotspice/core.py:56-980. See the module docstring for what runs where."""
 
@@ -828,10 +845,13 @@ class Magnets(ABC):
         if method == 'auto':
             method = 'igemm'
             if N * W <= self.engine.direct_max_pairs or not self._igemm_ok(d):
-                # FP64 either way. The direct sum walks a cell's window serially (about 0.2 us per
-                # entry), so up to 9 x 9 entries it is done before the convolution's three passes
-                # (200 x 200 cells, 5 x 5: 12 against 30 us; 128 x 128, 17 x 17: 55 against 26 us).
-                nfft = self._lib.hs_fft_scratch_bytes(L) if W > 81 else 0
+                # FP64 either way; the choice depends on the kernel set and the channels alone
+                plan = getattr(d, '_fft_plan', None)
+                if plan is None or plan[0] is not ks or plan[1] != self.USE_PERP_ENERGY:
+                    slots = ks.K.shape[0] if self.USE_PERP_ENERGY else (ks.K.shape[0] + 1) // 2
+                    nfft = self._lib.hs_fft_scratch_bytes(L) if fft_is_faster(N, self.n, W, slots, ks.wrap) else 0
+                    plan = d._fft_plan = (ks, self.USE_PERP_ENERGY, nfft)
+                nfft = plan[2]
                 method = 'fft64' if nfft > 0 else 'direct64'
         elif method == 'fft64':
             nfft = self._lib.hs_fft_scratch_bytes(L)
