@@ -842,7 +842,8 @@ class Magnets(ABC):
         N = self.nx * self.ny
         W = N if ks.full else (2 * ks.wx + 1) * (2 * ks.wy + 1)
         nfft = 0
-        if method == 'auto':
+        auto = method == 'auto'
+        if auto:
             method = 'igemm'
             if N * W <= self.engine.direct_max_pairs or not self._igemm_ok(d):
                 # FP64 either way; the choice depends on the kernel set and the channels alone
@@ -861,7 +862,13 @@ class Magnets(ABC):
             raise ValueError('igemm recompute needs the full uncropped kernel and a uniform moment')
         if method == 'fft64':
             # stream-ordered temporary: the allocator hands the memory on in this stream's order
-            tmp = torch.empty(nfft, device=self.device, dtype=torch.uint8)
+            try:
+                tmp = torch.empty(nfft, device=self.device, dtype=torch.uint8)
+            except torch.cuda.OutOfMemoryError:
+                if not auto:
+                    raise
+                method = 'direct64'        # the same sums without a temporary, more slowly
+        if method == 'fft64':
             _lib.check(self._lib.hs_dipolar_full_fft(L, tmp.data_ptr(), nfft, d._E.data_ptr(),
                                                      _ptr(d._Ep) if self.USE_PERP_ENERGY else None,
                                                      self._stream()), 'hs_dipolar_full_fft')

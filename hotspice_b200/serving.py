@@ -84,7 +84,9 @@ def geometry_shape(spec) -> tuple[int, int]:
 def footprint_bytes(spec) -> int:
     """Device bytes a request holds while resident (estimate made before it is built): per
     cell the spins, moments, FP64 energies (and perpendicular energies), E_B, temperature and
-    Zeeman factors, scratch; plus the kernel windows of the dipolar cutoff."""
+    Zeeman factors, scratch; plus the kernel windows of the dipolar cutoff. The temporary of a full
+    recompute is not among them: the allocator takes it back when memory runs short, and without it
+    the energies are summed directly."""
     ny, nx = geometry_shape(spec)
     cells = nx * ny
     per_cell = 96 if spec['lattice'] in ('IP_Pinwheel', 'IP_Kagome') else 64
