@@ -792,7 +792,7 @@ class Magnets(ABC):
 
     def _switch_list(self, cap):
         sl = getattr(self, '_sw', None)
-        if sl is None or sl[0].numel() < cap:
+        if sl is None or sl[1].cap < cap:
             cap = max(cap, 64)
             t = torch.zeros((3, cap), device=self.device, dtype=torch.int32)
             s = _lib.HsSwitchList()
