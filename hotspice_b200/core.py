@@ -797,6 +797,7 @@ class Magnets(ABC):
             t = torch.zeros((3, cap), device=self.device, dtype=torch.int32)
             s = _lib.HsSwitchList()
             s.y, s.x, s.mode, s.cap = t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), cap
+            s.tensor = t       # whoever keeps the pointers keeps the memory, also after the list has grown
             self._sw = (t, s)
             self._graphs.clear()
         return self._sw
