@@ -352,9 +352,9 @@ struct Sync {
     }
 };
 
-// Block minimum of (key, index); `warp_uniform`: v is already the warp's minimum on every lane.
-HS_DEV HsKeyIdx eng_block_kmin(HsKeyIdx v, HsKeyIdx *sm, bool warp_uniform = false) {
-    if (!warp_uniform) v = hs_warp_kmin(v);
+// Block minimum of (key, index).
+HS_DEV HsKeyIdx eng_block_kmin(HsKeyIdx v, HsKeyIdx *sm) {
+    v = hs_warp_kmin(v);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) sm[warp] = v;
     __syncthreads();
@@ -417,7 +417,7 @@ struct __align__(16) EngShared {
     HsKeyIdx part[2][16];               // owner path: the CTAs' minima of step st in part[st & 1]
     HsKeyIdx red[32];
     double dred[32];
-    int inst, n1, y1, x1, m1, nsw;
+    int inst, n1, y1, x1, nsw;
     int go[2];                          // step st runs while go[st & 1] (double-buffered)
     float mm1;
     double thr[2];                      // owner path: a key below thr[st & 1] switches for certain
@@ -1063,14 +1063,13 @@ HS_DEV void run_instance(EngShared &sh, const HsInstance *insts, int ii, int ran
                     S.publish(&sh.y1, flip.y);
                     S.publish(&sh.x1, flip.x);
                     S.publish(&sh.mm1, flip.mm_new);
-                    S.publish(&sh.m1, (int)flip.m_new);
                 }
                 decide_next(st + 1);
             }
             // The flip's global writes (spin, moment, switch list) are issued after this
             // thread's arrival at the barrier, so the barrier does not wait for them: the
-            // window update takes the switched cell's new spin and moment from the handover,
-            // and the writes are ordered before the next step by the barrier that ends this one.
+            // window update takes the switched cell's new moment from the handover, and the
+            // writes are ordered before the next step by the barrier that ends this one.
             S.all_then(rank == 0 && threadIdx.x == 0 && flip.flip, [&] { neel_apply(L, sw, flip); });
             if (L.has_dipolar && sh.n1 > 0)
                 update_one(L, sh.y1, sh.x1, sh.mm1, rank * blockDim.x + threadIdx.x, SCS * blockDim.x);

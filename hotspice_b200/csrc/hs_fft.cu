@@ -73,9 +73,6 @@ HS_DEV double2 mul_mi(double2 a) { return make_double2(a.y, -a.x); }     // -i a
 
 // Forward transforms of R values, natural order in and out.
 template <int R> struct Dft;
-template <> struct Dft<2> {
-    HS_DEV static void run(double2 *v) { const double2 a = v[0]; v[0] = cadd(a, v[1]); v[1] = csub(a, v[1]); }
-};
 template <> struct Dft<3> {
     HS_DEV static void run(double2 *v) {
         const double s = 0.86602540378443864676;   // sin(2 pi / 3)
