@@ -4,7 +4,10 @@
 //
 // is a correlation of the source field with each sublattice's window, so it costs three passes of
 // short transforms instead of one product per pair. All of it is FP64 from the FP32 kernels and
-// source field, as in the direct sum; the result differs from the direct sum's by FP64 rounding.
+// source field, as in the direct sum; the result differs from the direct sum's by FP64 rounding of the
+// largest sum the sources could give, about 2^-52 max|K| max|m mu| sqrt(magnets), where the direct
+// sum rounds relative to each cell's own terms. For two lone magnets 720 cells apart that is 1.5e-9 of
+// their energy, 2047 cells apart (2048 x 2 cells) 8e-7; the FP32 kernel values are off by 6e-8.
 //   fft_rows_kernel   transforms along x of the source rows and of every kernel row (reversed, so
 //                     that the correlation becomes a convolution)
 //   fft_cols_kernel   per column of the spectrum: transforms along y of the source and of each

@@ -244,9 +244,10 @@ class DipolarEnergy(Energy):
 
     def update(self, method: str | None = None):
         """Full recompute (hotspice/energies.py:290-308). ``method``: 'fft64' (FP64 fast
-        convolution, the default up to EngineConfig.direct_max_pairs cell pairs), 'direct64'
-        (FP64 direct sum, the default for windows of a few cells), 'direct32', or 'igemm'
-        (split-BF16 tensor-core implicit GEMM)."""
+        convolution), 'direct64' (FP64 direct sum), 'direct32', or 'igemm' (split-BF16 tensor-core
+        implicit GEMM). By default the faster of the first two up to EngineConfig.direct_max_pairs
+        cell pairs (core.fft_is_faster), 'igemm' beyond. 'fft64' rounds relative to the largest sum
+        the magnets could give, not to each cell's."""
         self.mm._full_recompute(self, method)
 
     def update_single(self, index2D):
