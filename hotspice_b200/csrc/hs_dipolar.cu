@@ -604,10 +604,10 @@ int hs_launch_dipolar_update(const HsLattice &L, const HsSwitchList &sw, const i
     // against 44 us of the persistent kernel). Uncut windows were measured when every switch still
     // visited the whole lattice (Poisson, 1024 x 1024: 162 against 17 us) and stay with those kernels.
     if (most <= FEW_MAX && items <= FEW_ITEMS) {
-        const int cap = std::max(most, 1);
-        const int grid = (int)std::min<int64_t>(2 * 148, (cap * items + FEW_T / 32 - 1) / (FEW_T / 32));
-        return hs_launch_step("dip_update_few_kernel", dip_update_few_kernel, grid, FEW_T, cap * sizeof(FewSw), st, L, sw, n_sw_dev,
-                              n_host, semantics, C, cap);
+        const int64_t room = std::max(most, 1);        // a list without room holds nothing to load
+        const int grid = (int)std::min<int64_t>(2 * 148, (room * items + FEW_T / 32 - 1) / (FEW_T / 32));
+        return hs_launch_step("dip_update_few_kernel", dip_update_few_kernel, grid, FEW_T, room * sizeof(FewSw), st, L, sw, n_sw_dev,
+                              n_host, semantics, C, most);
     }
     if (most <= UPD_PLOC && tiles <= 1 << 20 && tiles >= HS_UPD_PERSIST_MIN_TILES) {
         const int cap = std::max(most, 1);
